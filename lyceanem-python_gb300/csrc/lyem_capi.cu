@@ -62,6 +62,16 @@ __global__ void mask_to_bytes_kernel(const unsigned* __restrict__ bits, long lon
     }
 }
 
+// Clears the mask rows that src_order lists.
+__global__ void zero_mask_rows_kernel(unsigned* __restrict__ bits, const int* __restrict__ src_order, long long n_src,
+                                      long long words) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_src * words;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long k = i / words;
+        bits[src_order[k] * words + (i - k * words)] = 0u;
+    }
+}
+
 unsigned blocks_for(long long n, int threads) { return capped_blocks(n, threads, 32); }
 
 BinSpec grid_spec(const float* origin3, float cell, const int32_t* dims3) {
@@ -390,8 +400,17 @@ LYEM_API int lyem_pair_stage(const float* d_src_pos, const float* d_src_E, const
         p.refill_lanes = traversal == 0 ? -16 : traversal == 1 ? 0 : traversal <= 33 ? traversal - 1
                          : traversal == 38 ? -38 : kCapped[traversal - 34];
     }
-    if (d_mask_bits && d_snk_order)  // permuted sinks set their mask bits one by one
-        LYEM_CK(cudaMemsetAsync(d_mask_bits, 0, sizeof(uint32_t) * (size_t)n_src * (size_t)p.mask_words, s));
+    // permuted sinks, and the transposed schedule's warps, set their mask bits one by one
+    if (d_mask_bits && (d_snk_order || (use_grid && traversal == 38))) {
+        if (d_src_order) {  // (it may list any rows)
+            zero_mask_rows_kernel<<<blocks_for(n_src * p.mask_words, 256), 256, 0, s>>>(d_mask_bits, d_src_order, n_src,
+                                                                                       p.mask_words);
+            note_launches(1);
+            LYEM_CK(cudaGetLastError());
+        } else {
+            LYEM_CK(cudaMemsetAsync(d_mask_bits, 0, sizeof(uint32_t) * (size_t)n_src * (size_t)p.mask_words, s));
+        }
+    }
     LYEM_CK(launch_pair_stage(p, cull, s));
     if (d_sink_out) {
         const long long chunks = (n_src + chunk - 1) / chunk;

@@ -572,15 +572,32 @@ __global__ void __launch_bounds__(kThreads, MODE == kLockstep10 ? 10 : (MODE == 
 }
 
 // Transposed grid stage (traversal 38).  The lanes of a warp are the 32
-// sources of the block's chunk, and each warp traces its 32 sinks one after
-// the other, so the 32 rays a warp walks together end at the same sink.  When
+// sources of the block's chunk, and a warp traces them to one sink after the
+// other, so the 32 rays a warp walks together end at the same sink.  When
 // the sources are the elements of an array (millimetres apart) those rays cross
 // the same cells and test the same triangles, where a warp of the lockstep
 // schedule holds 32 directions from one source (a CPU model of the walk on the
 // 28 GHz scene: 78.5 instead of 124.8 test iterations per 32 array rays).  The
 // field of each sink is summed over the warp's lanes in a fixed butterfly order
 // and lane 0 writes the chunk's partial sum of that sink.
+//
+// A warp takes one to four sinks (transposed_sinks): the walk is bound by
+// latency, and a warp per sink gives the most warps and spreads neighbouring sinks,
+// whose rays share cells, over the warps of an SM.  256 elements, 120,000 triangles, 32 / 8 / 4 / 2 / 1 sinks a warp:
+// to 20,000 scatter points - / 1.05 / 0.91 / 0.85 / 0.81 ms (lockstep 2.08), to 4,186 sinks 1.23 / - / - / - / 0.28
+// (0.60); the two array stages of the 28 GHz scene (1,024 elements) 11.3 -> 10.1 and 8.2 -> 7.2 ms.  So few sinks do not pay
+// the search for a source's own-surface triangle that the lockstep schedule makes.
 constexpr int kTChunk = 32;
+
+// Sinks per warp of the transposed schedule: more than one only where the launch has far more warps than the GPU
+// holds (4,096 elements to 65,341 sinks: 33.6 / 33.0 / 32.8 / 34.5 ms with 1 / 2 / 4 / 8).
+static int transposed_sinks(long long n_src, long long n_snk) {
+    const long long chunks = (n_src + kTChunk - 1) / kTChunk;
+    const long long want = (long long)device_sm_count() * 4096;
+    int k = 4;
+    while (k > 1 && chunks * ((n_snk + k - 1) / k) < want) k /= 2;
+    return k;
+}
 
 template <bool CULL, bool WEIGHTED, bool PAIR_OUT, bool MASK_OUT, bool COUNT>
 __global__ void __launch_bounds__(kThreads, 16) grid_transposed_kernel(const StageParams p) {
@@ -591,26 +608,17 @@ __global__ void __launch_bounds__(kThreads, 16) grid_transposed_kernel(const Sta
     const int nsrc = (int)p.n_src - n0 < kTChunk ? (int)p.n_src - n0 : kTChunk;
     const bool n_ok = lane < nsrc;
     const int n = n_ok ? (p.src_order ? p.src_order[n0 + lane] : n0 + lane) : 0;
-    // each source's own-surface triangle (one warp per source), tried before the walk
-    __shared__ int s_hint[kTChunk];
-    for (int s = warp; s < nsrc; s += kThreads / 32) {
-        const int ns = p.src_order ? p.src_order[n0 + s] : n0 + s;
-        const float* so = p.src_pos + 3 * (long long)ns;
-        const int h = warp_nearest_ref(p, so[0], so[1], so[2]);
-        if (lane == 0) s_hint[s] = h;
-    }
-    __syncthreads();
+    const int spw = p.snk_per_warp;
     float ox = 0.f, oy = 0.f, oz = 0.f;
     if (n_ok) {
         const float* so = p.src_pos + 3 * (long long)n;
         ox = so[0]; oy = so[1]; oz = so[2];
     }
-    const int hint = n_ok ? s_hint[lane] : -1;
-    const int ms0 = (int)blockIdx.x * kThreads + warp * 32;  // the warp's first sink slot
+    const int ms0 = ((int)blockIdx.x * (kThreads / 32) + warp) * spw;  // the warp's first sink slot
     unsigned vis_mask = 0;                                    // bit k: this lane's source sees slot ms0 + k
     unsigned int tests = 0;
     Walk w;
-    for (int k = 0; k < 32; ++k) {
+    for (int k = 0; k < spw; ++k) {
         const int ms = ms0 + k;
         if (ms >= p.n_snk) break;  // the same in every lane
         const int m = p.snk_order ? p.snk_order[ms] : ms;
@@ -618,13 +626,8 @@ __global__ void __launch_bounds__(kThreads, 16) grid_transposed_kernel(const Sta
                     ez = p.snk_pos[3 * (long long)m + 2];
         bool vis = n_ok;  // untested pairs (the skipped diagonal, segments off the grid) are visible
         if (n_ok && !(p.skip_diag && n == m)) {
-            walk_ray<CULL>(w, ox, oy, oz, ex, ey, ez);
             bool hit = false;
-            if (hint >= 0) {
-                if (COUNT) ++tests;
-                hit = walk_test_ref<CULL>(p, w, hint);
-            }
-            if (!hit && walk_setup(p, w)) {
+            if (walk_begin<CULL>(p, w, ox, oy, oz, ex, ey, ez)) {
                 while (!hit) {
                     while (w.q < w.q1) {
                         if (COUNT) ++tests;
@@ -657,7 +660,10 @@ __global__ void __launch_bounds__(kThreads, 16) grid_transposed_kernel(const Sta
         }
     }
     if (n_ok) {
-        if (MASK_OUT && !p.snk_order && ms0 < p.n_snk) p.mask_bits[(long long)n * p.mask_words + (ms0 >> 5)] = vis_mask;
+        if (MASK_OUT && !p.snk_order && ms0 < p.n_snk) {
+            if (vis_mask)  // (mask zeroed by the host)
+                atomicOr(p.mask_bits + (long long)n * p.mask_words + (ms0 >> 5), vis_mask << (ms0 & 31));
+        }
         if (p.src_visible && vis_mask) atomicAdd(p.src_visible + n, __popc(vis_mask));
     }
     if (p.counters) {
@@ -701,6 +707,8 @@ static cudaError_t launch_t(const StageParams& p0, cudaStream_t stream) {
                 else
                     grid_stage_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, kTwoPhase12><<<grid, kThreads, qbytes, stream>>>(p);
             } else if (p.refill_lanes == -38) {
+                p.snk_per_warp = transposed_sinks(p.n_src, p.n_snk);
+                grid.x = (unsigned)((p.n_snk + p.snk_per_warp * (kThreads / 32) - 1) / (p.snk_per_warp * (kThreads / 32)));
                 if (p.counters)
                     grid_transposed_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, true><<<grid, kThreads, 0, stream>>>(p);
                 else

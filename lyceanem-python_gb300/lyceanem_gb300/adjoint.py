@@ -47,7 +47,7 @@ class SinkField(torch.autograd.Function):
             r1 = P.pair_stage(x, E_src, scat, scat_n, snk_order=order, traversal=ts, **kw)
             w = r1.sink
             r2 = P.pair_stage(scat, w, y, snk_n, src_W=w, sink_out=E, accumulate=True, src_order=order,
-                              snk_order=o_snk, **kw)
+                              snk_order=o_snk, traversal=P.scatter_schedule(M, grid), **kw)
             masks = (r0.mask_bits, r1.mask_bits, r2.mask_bits)
         else:
             scat = scat_n = w = None

@@ -41,12 +41,12 @@ def form_network(src, pol, snk, snk_n, *, beta, alpha=0.0, grid=None, tris=None,
     """Propagation network complex64 [N, M, 3] for unit element excitations pol (complex [3] or [N,3]),
     optionally scaled per element by `weights` (e.g. element areas).  self_to_self=True tests every pair;
     False reproduces the reference engine's untested pair n == m."""
-    src = P._points(src)
+    src, snk = P._points(src), P._points(snk)
     E = P._cvec(pol, src.shape[0])
     if weights is not None:
         E = E * P._dev(weights, torch.complex64).reshape(-1, 1)
     return P.pair_stage(src, E, snk, snk_n, beta=beta, alpha=alpha, grid=grid, tris=tris, want_pairs=True,
-                        self_to_self=self_to_self).pairs
+                        self_to_self=self_to_self, traversal=P.source_schedule(src, grid, snk.shape[0])).pairs
 
 
 class BeamSweep:

@@ -89,7 +89,8 @@ class _DeviceScene:
         E = _cvec_from_point_data(source_mesh)
         out = np.zeros((src.shape[0], snk.shape[0], 3), dtype=np.complex64)
         for a, b in _chunks(src.shape[0], chunk_count):
-            r = self.stage(src[a:b], E[a:b], snk, snk_n, alpha, beta, self_to_self, want_pairs=True)
+            r = self.stage(src[a:b], E[a:b], snk, snk_n, alpha, beta, self_to_self, want_pairs=True,
+                           traversal=P.source_schedule(src[a:b], self.grid))
             out[a:b] = r.pairs.cpu().numpy()
         return out
 

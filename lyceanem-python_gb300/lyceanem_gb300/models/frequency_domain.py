@@ -70,6 +70,7 @@ def sink_field(structure, src, E, snk, snk_n, alpha, beta, scat=None, scat_n=Non
     o_snk = _sink_order(dev, snk)
     # the stages that start at the sources take the transposed schedule when the sources are compact (an array)
     ts = P.source_schedule(src, dev.grid)
+    tp = P.scatter_schedule(snk.shape[0], dev.grid)
     out = P.pair_stage(src, E, snk, snk_n, snk_order=o_snk, traversal=ts, **kw).sink
     if scattering >= 1 and scat is not None and len(scat):
         scat = P._points(scat)
@@ -77,7 +78,7 @@ def sink_field(structure, src, E, snk, snk_n, alpha, beta, scat=None, scat_n=Non
         if not skip_unlit:
             e_p = P.pair_stage(src, E, scat, scat_n, snk_order=o_scat, traversal=ts, **kw).sink
             P.pair_stage(scat, e_p, snk, snk_n, src_W=e_p, sink_out=out, accumulate=True, src_order=o_scat,
-                         snk_order=o_snk, **kw)
+                         snk_order=o_snk, traversal=tp, **kw)
             return out
         seen = torch.zeros(scat.shape[0], dtype=torch.int32, device=scat.device)
         e_p = P.pair_stage(src, E, scat, scat_n, snk_order=o_scat, traversal=ts, snk_visible=seen, **kw).sink
@@ -86,7 +87,7 @@ def sink_field(structure, src, E, snk, snk_n, alpha, beta, scat=None, scat_n=Non
         lit = o_scat[seen[o_scat.long()] > 0].contiguous()
         if lit.numel():
             P.pair_stage(scat, e_p, snk, snk_n, src_W=e_p, sink_out=out, accumulate=True, src_order=lit,
-                         snk_order=o_snk, **kw)
+                         snk_order=o_snk, traversal=tp, **kw)
     return out
 
 
@@ -158,8 +159,9 @@ def numba_sink_field(structure, src, E, snk, snk_n, alpha, beta, scat=None, scat
     snk_n_t = P._points(snk_n)
     snk = P._points(snk)
     o_snk = _sink_order(dev, snk)
+    ts = P.source_schedule(src, dev.grid)
     if scattering == 0 or los:
-        out = P.pair_stage(src, E, snk, snk_n_t, snk_order=o_snk, **kw).sink
+        out = P.pair_stage(src, E, snk, snk_n_t, snk_order=o_snk, traversal=ts, **kw).sink
     else:
         out = torch.zeros((snk_n_t.shape[0], 3), dtype=torch.complex64, device=snk_n_t.device)
     if scattering >= 1:
@@ -167,9 +169,10 @@ def numba_sink_field(structure, src, E, snk, snk_n, alpha, beta, scat=None, scat
         if scat is not None and len(scat):
             scat_t = P._points(scat)
             o = P.spatial_order(scat_t)
-            e_p = P.pair_stage(src, E, scat_t, scat_n, snk_order=o, **kw).sink
+            e_p = P.pair_stage(src, E, scat_t, scat_n, snk_order=o, traversal=ts, **kw).sink
             tangential_project(e_p, scat_n)
-            P.pair_stage(scat_t, e_p, snk, snk_n_t, sink_out=out, accumulate=True, src_order=o, snk_order=o_snk, **kw)
+            P.pair_stage(scat_t, e_p, snk, snk_n_t, sink_out=out, accumulate=True, src_order=o, snk_order=o_snk,
+                         traversal=P.scatter_schedule(snk.shape[0], dev.grid), **kw)
     return out
 
 
@@ -183,8 +186,9 @@ def numba_per_element(structure, src, E, snk, snk_n, alpha, beta, scat=None, sca
               eps=P.NUMBA_EPSILON, want_pairs=True)
     src_t, snk_t, snk_n_t = P._points(src), P._points(snk), P._points(snk_n)
     N, M = src_t.shape[0], snk_t.shape[0]
+    ts = P.source_schedule(src, dev.grid)
     if scattering == 0 or los:
-        S = P.pair_stage(src_t, E, snk_t, snk_n_t, **kw).pairs
+        S = P.pair_stage(src_t, E, snk_t, snk_n_t, traversal=ts, **kw).pairs
     else:
         S = torch.zeros((N, M, 3), dtype=torch.complex64, device=src_t.device)
     if scattering >= 1:
@@ -193,7 +197,7 @@ def numba_per_element(structure, src, E, snk, snk_n, alpha, beta, scat=None, sca
         if scat is not None and len(scat):
             scat_t, scat_n_t = P._points(scat), P._points(scat_n)
             Pn = scat_t.shape[0]
-            U = P.pair_stage(src_t, E, scat_t, scat_n_t, **kw).pairs
+            U = P.pair_stage(src_t, E, scat_t, scat_n_t, traversal=ts, **kw).pairs
             up = _unit(scat_n_t).to(torch.complex64)[None]
             U = U - (U * up).sum(-1, keepdim=True) * up
             for k in range(3):

@@ -471,6 +471,33 @@ def test_edge_sizes(n_src, n_snk, n_tris):
     _no_device_errors()
 
 
+@pytest.mark.parametrize("n_src,n_snk", [(1, 1), (31, 3), (33, 5), (65, 130), (2080, 20011)])
+@pytest.mark.parametrize("ordered", [False, True])
+def test_transposed_schedule_sinks_per_warp(n_src, n_snk, ordered):
+    """The transposed schedule at the edges of its sinks per warp (one, and two where the launch has enough warps) and
+    of its chunks of 32 sources: masks, visible counts and, with a subset of the sources, the rows left out."""
+    P = _P()
+    src, snk, snk_n, v, f, E = random_scene(n_src + n_snk, n_src=n_src, n_snk=n_snk, n_tris=40)
+    g = P.UniformGrid(P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f)))
+    o = P.direction_order(snk, g.centre) if ordered else None
+    kw = dict(beta=30.0, grid=g, want_mask=True, snk_order=o)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    res = []
+    for trav in (36, 38):
+        sv, kv = torch.zeros(n_src, **i32), torch.zeros(n_snk, **i32)
+        res.append((P.pair_stage(src, E, snk, snk_n, traversal=trav, src_visible=sv, snk_visible=kv, **kw), sv, kv))
+    (a, sa, ka), (b, sb, kb) = res
+    assert torch.equal(a.mask_bits, b.mask_bits) and torch.equal(sa, sb) and torch.equal(ka, kb)
+    assert rel_err(b.sink.cpu().numpy(), a.sink.cpu().numpy()) < 2e-6  # FP32 sums of up to 2,080 terms in two orders
+    if n_src > 1:  # every second row, from the last one down
+        sub = torch.arange(n_src - 1, -1, -2, **i32)
+        r = P.pair_stage(src, E, snk, snk_n, traversal=38, src_order=sub, **kw)
+        rows = torch.zeros(n_src, dtype=torch.bool, device="cuda")
+        rows[sub.long()] = True
+        assert torch.equal(r.mask_bits[rows], a.mask_bits[rows]) and not r.mask_bits[~rows].any()
+    _no_device_errors()
+
+
 def test_stage_buffer_checks():
     """Caller buffers of the wrong type or length are refused before any launch (the kernels index them
     without bounds checks)."""

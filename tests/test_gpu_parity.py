@@ -498,6 +498,23 @@ def test_transposed_schedule_sinks_per_warp(n_src, n_snk, ordered):
     _no_device_errors()
 
 
+@pytest.mark.parametrize("n", [1, 31, 33, 1025, 4096, 4097, 16384, 16385])
+def test_spatial_order_is_the_stable_morton_sort(n):
+    """Both sorts behind the orders (one block up to 16,384 points, passes of kernels above), at their edges, against
+    numpy's stable sort of the same Z-order keys; many equal keys (points on a coarse lattice)."""
+    P = _P()
+    rng = np.random.default_rng(n)
+    pts = rng.integers(0, 9, size=(n, 3)).astype(np.float32)
+    lo, ext = pts.min(0), pts.max(0) - pts.min(0)
+    sc = np.where(ext > 0, np.float32(1023) / np.where(ext > 0, ext, 1), 0).astype(np.float32)
+    q = ((pts - lo) * sc).astype(np.uint64)
+    key = np.zeros(n, np.uint64)
+    for b in range(10):
+        for k in range(3):
+            key |= ((q[:, k] >> np.uint64(b)) & np.uint64(1)) << np.uint64(3 * b + k)
+    assert np.array_equal(P.spatial_order(pts).cpu().numpy(), np.argsort(key, kind="stable"))
+
+
 def test_stage_buffer_checks():
     """Caller buffers of the wrong type or length are refused before any launch (the kernels index them
     without bounds checks)."""

@@ -133,6 +133,9 @@ LYEM_API size_t lyem_spatial_order_workspace(int64_t n_points);
  * Workspace: lyem_spatial_order_workspace(n_points) bytes. */
 LYEM_API int lyem_direction_order(const float *d_points, int64_t n_points, const float *centre3, int32_t *d_order,
                                   void *d_ws, size_t ws_bytes, void *stream);
+/* The same seen from a point in device memory (3 floats, e.g. a source's position). */
+LYEM_API int lyem_direction_order_from(const float *d_points, int64_t n_points, const float *d_centre3,
+                                       int32_t *d_order, void *d_ws, size_t ws_bytes, void *stream);
 LYEM_API int lyem_spatial_order(const float *d_points, int64_t n_points, int32_t *d_order, void *d_ws,
                                 size_t ws_bytes, void *stream);
 

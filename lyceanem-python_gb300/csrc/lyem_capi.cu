@@ -301,7 +301,18 @@ LYEM_API int lyem_direction_order(const float* d_points, int64_t n_points, const
         if (!isfinite(centre3[k])) return LYEM_ERR_INVALID;
     if (n_points >= (1LL << 31) - 64) return LYEM_ERR_OVERFLOW;
     if (!d_ws || ws_bytes < spatial_order_workspace_bytes(n_points)) return LYEM_ERR_WORKSPACE;
-    LYEM_CK(direction_order(d_points, n_points, centre3, d_order, d_ws, as_stream(stream)));
+    LYEM_CK(direction_order(d_points, n_points, centre3, nullptr, d_order, d_ws, as_stream(stream)));
+    return LYEM_OK;
+}
+
+LYEM_API int lyem_direction_order_from(const float* d_points, int64_t n_points, const float* d_centre3,
+                                       int32_t* d_order, void* d_ws, size_t ws_bytes, void* stream) {
+    if (n_points < 0) return LYEM_ERR_INVALID;
+    if (n_points == 0) return LYEM_OK;
+    if (!d_points || !d_order || !d_centre3) return LYEM_ERR_INVALID;
+    if (n_points >= (1LL << 31) - 64) return LYEM_ERR_OVERFLOW;
+    if (!d_ws || ws_bytes < spatial_order_workspace_bytes(n_points)) return LYEM_ERR_WORKSPACE;
+    LYEM_CK(direction_order(d_points, n_points, nullptr, d_centre3, d_order, d_ws, as_stream(stream)));
     return LYEM_OK;
 }
 

@@ -631,9 +631,12 @@ __global__ void morton_kernel(const float* __restrict__ pts, long long n, const 
 // tile) and points within a tile by 6-bit (elevation, azimuth) positions.
 // nb * na < 2^18 keeps keys below 2^30.
 __global__ void direction_key_kernel(const float* __restrict__ pts, long long n, float cx, float cy, float cz,
-                                     float tile, int nb, int na, int* keys, int* vals) {
+                                     const float* __restrict__ centre, float tile, int nb, int na, int* keys, int* vals) {
     const float kPi = 3.14159265358979f;
     const float inv = 1.f / tile;
+    if (centre) {
+        cx = centre[0]; cy = centre[1]; cz = centre[2];
+    }
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float dx = pts[3 * i] - cx, dy = pts[3 * i + 1] - cy, dz = pts[3 * i + 2] - cz;
         const float fe = (atan2f(dz, hypotf(dx, dy)) + 0.5f * kPi) * inv + 0.125f;
@@ -651,8 +654,8 @@ __global__ void direction_key_kernel(const float* __restrict__ pts, long long n,
     }
 }
 
-cudaError_t direction_order(const float* pts, long long n, const float* centre3, int* order, void* ws,
-                            cudaStream_t stream) {
+cudaError_t direction_order(const float* pts, long long n, const float* centre3, const float* d_centre3, int* order,
+                            void* ws, cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
     int* k0 = static_cast<int*>(ws) + 64;
     int* v0 = k0 + n + 64;
@@ -667,8 +670,9 @@ cudaError_t direction_order(const float* pts, long long n, const float* centre3,
     const double kPi = 3.14159265358979323846;
     const double tile = std::max(0.009, 4.0 * std::sqrt(2.0 * kPi * kPi / (double)n));
     const int nb = (int)std::ceil(kPi / tile) + 2, na = (int)std::ceil(2.0 * kPi / tile) + 2;
-    direction_key_kernel<<<b, 256, 0, stream>>>(pts, n, centre3[0], centre3[1], centre3[2], (float)tile,
-                                                          nb, na, k0, v0);
+    const float zero3[3] = {0.f, 0.f, 0.f};
+    const float* c = centre3 ? centre3 : zero3;
+    direction_key_kernel<<<b, 256, 0, stream>>>(pts, n, c[0], c[1], c[2], d_centre3, (float)tile, nb, na, k0, v0);
     note_launches(1);
     bool first = true;
     cudaError_t e = radix_sort_pairs(k0, v0, k1, order, n, (nb * na) << 12, hist, hist_scanned, scan_ws, &first, stream);

@@ -9,13 +9,11 @@
 // network (the reference's output layout) and a visibility bit mask.
 //
 // Brute force (replaces raycast_brute_force, lyceanem/src/raycasting_brute_force.cuh:68-88):
-// triangle tiles of 64 are staged in shared memory by TMA bulk copies
-// (double-buffered, mbarrier-completed, bounded waits); for each source of
-// the chunk the block derives the ray-independent part of the test once per
-// triangle (tvec, qvec, e2.qvec) and every thread tests its ray against the
-// tile.  A ray stops at its first hit; a tile step is skipped when no thread
-// of the block still has an unresolved ray (block vote), and the block stops
-// loading tiles once every ray is resolved.
+// triangle tiles of 128 are staged in shared memory by TMA bulk copies
+// (double-buffered, mbarrier-completed, bounded waits).  For each source of the chunk a warp takes 32
+// triangles at a time, a lane each: it derives the ray-independent part of the test (tvec, qvec, e2.qvec) and drops
+// the triangles that face away from the source or that the beam of the warp's 32 rays cannot meet; its rays then test
+// the others.  A ray stops at its first hit, and the block stops loading tiles once every ray is resolved.
 //
 // Grid (replaces raycast_tiles + DDA, lyceanem/src/raycasting_accelerated.cuh:106-268, 458-482):
 // each thread walks its segment through a uniform 3-D grid (Amanatides-Woo,
@@ -120,10 +118,9 @@ cudaError_t read_clear_device_errors(unsigned int* flags, cudaStream_t stream) {
 }
 
 constexpr int kThreads = 128;
-// Brute-force triangle tile: 64 triangles (3 KB raw + 4 KB derived per buffer)
-// leave room for more resident blocks than 128 did (8-array direct scene
-// 0.336 -> 0.277 ms; 32 measured 0.297 ms).
-constexpr int kTile = 64;
+// Brute-force triangle tile (a power of two; two block barriers a tile): 32 / 64 / 128 / 256 / 512 triangles measured
+// 0.270 / 0.256 / 0.240 / 0.275 / 0.327 ms on the 8 x 8-array direct scene.
+constexpr int kTile = 128;
 constexpr int kBruteMaxChunk = 32;  // one bit per source in a 32-bit mask
 constexpr int kGridMaxChunk = 64;   // one bit per source in a 64-bit mask
 
@@ -134,7 +131,7 @@ int transposed_src_chunk() { return 32; }
 
 struct BruteSmem {
     float4 raw[2][kTile * 3];
-    TriPre pre[2][kTile];
+    TriPre pre[kThreads / 32][32];  // a warp's candidates of the current 32 triangles
     unsigned long long mbar[2];
 };
 
@@ -221,16 +218,108 @@ __device__ __forceinline__ void flush_block(const StageParams& p, long long m, b
     }
 }
 
-// Registers capped so that 9 blocks fit an SM (56 registers, almost no spill):
-// the direct scene's 1,344 blocks then run in one wave on 152 SMs instead of
-// 8 per SM plus a tail (stage 0.266 -> 0.219 ms; a cap for 12 blocks spills
-// and measured 0.268 ms).
+// The warp's rays from one source as a beam: directions are multiples of (1, sy, sz) in the axes (x, y, z) = (k, k + 1,
+// k + 2 mod 3) with x mirrored by `sign`, sy in [y0, y1], sz in [z0, z1]; they end before x = far.
+struct BruteBeam {
+    int k;  // -1: rays too far apart, no beam
+    float sign, y0, y1, z0, z1, far;
+};
+
+__device__ __forceinline__ float axis_of(int k, float x, float y, float z) { return k == 0 ? x : k == 1 ? y : z; }
+
+__device__ __forceinline__ float redux_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float redux_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Beam of the rays of the lanes with `open` (at least one).  A ray without a direction (coincident or non-finite end
+// points) hits nothing and is left out.
+__device__ __forceinline__ BruteBeam brute_beam(const Ray& r, bool open) {
+    const unsigned full = 0xffffffffu;
+    BruteBeam b;
+    open = open && r.dx * r.dx + r.dy * r.dy + r.dz * r.dz > 0.5f;
+    const unsigned who = __ballot_sync(full, open);
+    // the axis that the rays' common part is longest along
+    const float ax = fmaxf(redux_min(open ? r.dx : 2.f), -redux_max(open ? r.dx : -2.f));
+    const float ay = fmaxf(redux_min(open ? r.dy : 2.f), -redux_max(open ? r.dy : -2.f));
+    const float az = fmaxf(redux_min(open ? r.dz : 2.f), -redux_max(open ? r.dz : -2.f));
+    const float m = fmaxf(ax, fmaxf(ay, az));
+    b.k = -1;
+    if (!who || !(m > 0.15f)) return b;
+    b.k = ax == m ? 0 : ay == m ? 1 : 2;
+    const int lead = __ffs(who) - 1;
+    b.sign = copysignf(1.f, __shfl_sync(full, axis_of(b.k, r.dx, r.dy, r.dz), lead));
+    const float x = axis_of(b.k, r.dx, r.dy, r.dz) * b.sign, inv = 1.f / x;
+    const float sy = axis_of(b.k, r.dy, r.dz, r.dx) * inv, sz = axis_of(b.k, r.dz, r.dx, r.dy) * inv;
+    const float y = __shfl_sync(full, sy, lead), z = __shfl_sync(full, sz, lead);
+    // widened by far more than the rounding of the slopes
+    b.y0 = redux_min(open ? sy : y) - 0x1p-16f;
+    b.y1 = redux_max(open ? sy : y) + 0x1p-16f;
+    b.z0 = redux_min(open ? sz : z) - 0x1p-16f;
+    b.z1 = redux_max(open ? sz : z) + 0x1p-16f;
+    b.far = redux_max(open ? r.len * x : 0.f) * 1.001f;
+    return b;
+}
+
+// Whether no ray of the beam from o can hit the triangle.  With t = o - v0 the test's numerators are linear in the ray
+// direction D: u = D.(e2 x t), v = D.(t x e1), A = D.(e2 x e1), and w = -t.(e2 x e1).  A hit has u, v, A - u - v >= 0 and
+// 0 < w < A len (two-sided: all by A's sign) to within FP32 rounding, so the triangle is missed when one of them fails
+// over the whole slope rectangle by more than `slack`: the rounding of the test's and of this evaluation, for
+// directions scaled to x = 1, is below 2^-19 (1 + |sy| + |sz|) times the product of the vectors' 1-norms.
+template <bool CULL>
+__device__ __forceinline__ bool beam_misses(const BruteBeam& B, const TriPre& p) {
+    const int k = B.k;
+    const float tx = axis_of(k, p.b.z, p.b.w, p.c.x), ty = axis_of(k, p.b.w, p.c.x, p.b.z), tz = axis_of(k, p.c.x, p.b.z, p.b.w);
+    const float ax = axis_of(k, p.a.x, p.a.y, p.a.z), ay = axis_of(k, p.a.y, p.a.z, p.a.x), az = axis_of(k, p.a.z, p.a.x, p.a.y);
+    const float bx = axis_of(k, p.a.w, p.b.x, p.b.y), by = axis_of(k, p.b.x, p.b.y, p.a.w), bz = axis_of(k, p.b.y, p.a.w, p.b.x);
+    const float na = fabsf(ax) + fabsf(ay) + fabsf(az), nb = fabsf(bx) + fabsf(by) + fabsf(bz);
+    const float nt = fabsf(tx) + fabsf(ty) + fabsf(tz);
+    const float smax = fmaxf(fabsf(B.y0), fabsf(B.y1)) + fmaxf(fabsf(B.z0), fabsf(B.z1));
+    const float slack = (0x1p-19f + 0x1p-19f * smax) * (nt + na) * (na + nb);
+    // gradients of u, v and A (cyclic axes keep the cross products), x mirrored with the beam
+    float ux = (by * tz - bz * ty) * B.sign, uy = bz * tx - bx * tz, uz = bx * ty - by * tx;
+    float vx = (ty * az - tz * ay) * B.sign, vy = tz * ax - tx * az, vz = tx * ay - ty * ax;
+    const float nx = by * az - bz * ay;
+    float cx = nx * B.sign, cy = bz * ax - bx * az, cz = bx * ay - by * ax;
+    float w = -(tx * nx + ty * cy + tz * cz);
+    const float ym = 0.5f * (B.y0 + B.y1), zm = 0.5f * (B.z0 + B.z1), yh = B.y1 - ym, zh = B.z1 - zm;
+    float am = cx + ym * cy + zm * cz;
+    const float ah = yh * fabsf(cy) + zh * fabsf(cz) + slack;
+    if (!CULL) {  // the sign of A has to be the same over the beam
+        const float s = am < 0.f ? -1.f : 1.f;
+        am = fabsf(am);
+        if (!(am > ah)) return false;
+        ux *= s; uy *= s; uz *= s;
+        vx *= s; vy *= s; vz *= s;
+        cx *= s; cy *= s; cz *= s;
+        w *= s;
+    }
+    cx -= ux + vx; cy -= uy + vy; cz -= uz + vz;
+    const float amax = am + ah, ws = slack * nt;
+    return amax < 0.f || w < -ws || w > amax * B.far + ws ||
+           ux + ym * uy + zm * uz + yh * fabsf(uy) + zh * fabsf(uz) < -slack ||
+           vx + ym * vy + zm * vz + yh * fabsf(vy) + zh * fabsf(vz) < -slack ||
+           cx + ym * cy + zm * cz + yh * fabsf(cy) + zh * fabsf(cz) < -slack;
+}
+
+// Registers capped so that 9 blocks fit an SM: the 8 x 8-array direct scene's 1,344 blocks then run in one wave on 152
+// SMs.  Bound by the FP32 work of the per-triangle part, which every warp does for its own beam (about 180 instructions per 32
+// triangles).  Against tests of every triangle by every ray: 64 sources, 2,664 sinks, 1,024 triangles 0.279 -> 0.240 ms
+// with the sinks in their natural order, 0.161 in direction order (two-sided test 0.620 -> 0.447 / 0.277); 256 sources,
+// 16,380 sinks 3.89 -> 1.67 / 1.23.
 template <bool CULL, bool WEIGHTED, bool PAIR_OUT, bool MASK_OUT>
 __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StageParams p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     BruteSmem& sm = *reinterpret_cast<BruteSmem*>(smem_raw);
 
-    const int tid = threadIdx.x;
+    const unsigned full = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31;
     const long long ms = (long long)blockIdx.x * kThreads + tid;
     const bool m_ok = ms < p.n_snk;
     const long long m = m_ok ? (p.snk_order ? (long long)p.snk_order[ms] : ms) : 0;
@@ -241,10 +330,9 @@ __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StagePar
         return p.src_order ? (long long)p.src_order[n0 + s] : n0 + s;
     };
 
-    float ex = 0.f, ey = 0.f, ez = 0.f, nx = 0.f, ny = 0.f, nz = 0.f;
+    float ex = 0.f, ey = 0.f, ez = 0.f;
     if (m_ok) {
         ex = p.snk_pos[3 * m]; ey = p.snk_pos[3 * m + 1]; ez = p.snk_pos[3 * m + 2];
-        nx = p.snk_nrm[3 * m]; ny = p.snk_nrm[3 * m + 1]; nz = p.snk_nrm[3 * m + 2];
     }
     uint32_t pending = 0, blocked = 0;
     for (int s = 0; s < nsrc; ++s)
@@ -264,68 +352,94 @@ __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StagePar
         long long cnt = T - first < kTile ? T - first : kTile;
         tma_load_1d(smem_addr(&sm.raw[k & 1][0]), p.tris + 3 * first, (uint32_t)(cnt * 48), (k & 1) ? mb1 : mb0);
     };
-    if (tid == 0) {
-        if (ntiles > 0) issue(0);
-        if (ntiles > 1) issue(1);
-    }
+    int issued = ntiles < 2 ? ntiles : 2;
+    if (tid == 0)
+        for (int k = 0; k < issued; ++k) issue(k);
 
     unsigned long long tests = 0;
     bool timed_out = false;
     // with one source per block (the automatic shape for few sources) the lane's
-    // ray is formed once instead of once per tile
+    // ray and the warp's beam are formed once instead of once per tile
     Ray r1 = Ray{0.f, 0.f, 0.f, 0.f};
-    if (nsrc == 1 && (pending & 1u)) {
+    BruteBeam b1;
+    b1.k = -1;
+    if (nsrc == 1) {
         const float* so = p.src_pos + 3 * src_index(0);
         r1 = vis_ray<CULL>(so[0], so[1], so[2], ex, ey, ez);
+        b1 = brute_beam(r1, pending & 1u);
     }
+    TriPre* pre = sm.pre[tid >> 5];
     int k = 0;
     for (; k < ntiles; ++k) {
         if (!__syncthreads_or(pending != 0)) break;
+        // the vote is a barrier: tile k - 1 has been read by every thread, and its buffer takes tile k + 1
+        if (k >= 1 && issued == k + 1 && issued < ntiles) {
+            if (tid == 0) {
+                fence_proxy_async_smem();
+                issue(issued);
+            }
+            ++issued;
+        }
         bool ok = mbar_wait_bounded((k & 1) ? mb1 : mb0, (k >> 1) & 1, kWaitCycles);
         if (__syncthreads_or(!ok)) { timed_out = true; break; }
         const int cnt = (int)(T - (long long)k * kTile < kTile ? T - (long long)k * kTile : kTile);
         const float4* rt = sm.raw[k & 1];
         for (int s = 0; s < nsrc; ++s) {
-            TriPre* pb = sm.pre[(k * nsrc + s) & 1];
+            bool open = (pending >> s) & 1u;
+            if (!__any_sync(full, open)) continue;
             const float* so = p.src_pos + 3 * src_index(s);
             const float ox = so[0], oy = so[1], oz = so[2];
-            if (tid < cnt) pb[tid] = make_tripre(ox, oy, oz, rt[3 * tid], rt[3 * tid + 1], rt[3 * tid + 2]);
-            const bool mine = (pending >> s) & 1u;
-            if (!__syncthreads_or(mine)) continue;
-            if (mine) {
-                const Ray r = nsrc == 1 ? r1 : vis_ray<CULL>(ox, oy, oz, ex, ey, ez);
-                int j = 0;
-                bool hitany = false;
-                for (; j < cnt; ++j) {
-                    if (hit_pre<CULL>(r, pb[j], p.eps)) { hitany = true; break; }
-                }
-                tests += hitany ? (unsigned long long)(j + 1) : (unsigned long long)cnt;
-                if (hitany) {
-                    pending &= ~(1u << s);
-                    blocked |= 1u << s;
-                }
+            Ray r = r1;
+            BruteBeam beam = b1;
+            if (nsrc > 1) {
+                r = vis_ray<CULL>(ox, oy, oz, ex, ey, ez);
+                beam = brute_beam(r, open);
             }
-        }
-        // Every thread has finished reading raw[k & 1] (the block vote of the
-        // last source step above is a barrier): refill it with tile k + 2.
-        if (tid == 0 && k + 2 < ntiles) {
-            fence_proxy_async_smem();
-            issue(k + 2);
+            for (int base = 0; base < cnt; base += 32) {
+                const int j = base + lane;
+                bool keep = j < cnt;
+                if (keep) {
+                    const TriPre t = make_tripre(ox, oy, oz, rt[3 * j], rt[3 * j + 1], rt[3 * j + 2]);
+                    // culling test: w = e2.qvec not positive is a miss for every ray, bit for bit (cull_tail)
+                    if (CULL) keep = t.d.x > 0.f;
+                    if (keep && beam.k >= 0) keep = !beam_misses<CULL>(beam, t);
+                    if (keep) pre[lane] = t;
+                }
+                unsigned cand = __ballot_sync(full, keep);
+                __syncwarp();
+                while (cand) {
+                    const int c = __ffs(cand) - 1;
+                    cand &= cand - 1;
+                    if (open && hit_pre<CULL>(r, pre[c], p.eps)) {
+                        open = false;
+                        tests += c + 1;  // (a dropped triangle counts as tested: the ray's outcome is decided)
+                    }
+                }
+                if (open) tests += cnt - base < 32 ? cnt - base : 32;
+                if (!__any_sync(full, open)) break;
+                __syncwarp();
+            }
+            if (!open && ((pending >> s) & 1u)) {
+                pending &= ~(1u << s);
+                blocked |= 1u << s;
+            }
+            __syncwarp();
         }
     }
     // Wait (bounded) for copies still in flight before the block may exit.
-    {
-        int hi = k + 2 < ntiles ? k + 2 : ntiles;
-        for (int j = k; j < hi; ++j) {
-            if (timed_out && j == k) continue;
-            if (!mbar_wait_bounded((j & 1) ? mb1 : mb0, (j >> 1) & 1, kWaitCycles)) timed_out = true;
-        }
+    for (int j = k; j < issued; ++j) {
+        if (timed_out && j == k) continue;
+        if (!mbar_wait_bounded((j & 1) ? mb1 : mb0, (j >> 1) & 1, kWaitCycles)) timed_out = true;
     }
     if (timed_out) {
         if (tid == 0) atomicOr(&g_device_error, 1u);
         return;
     }
 
+    float nx = 0.f, ny = 0.f, nz = 0.f;
+    if (m_ok) {
+        nx = p.snk_nrm[3 * m]; ny = p.snk_nrm[3 * m + 1]; nz = p.snk_nrm[3 * m + 2];
+    }
     float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     unsigned long long vis_count = 0;
     for (int s = 0; s < nsrc; ++s) {
@@ -680,13 +794,31 @@ __global__ void __launch_bounds__(kThreads, 16) grid_transposed_kernel(const Sta
     }
 }
 
-__global__ void reduce_partials_kernel(const float* __restrict__ partial, long long n_chunks, long long n_elem,
-                                       float* __restrict__ out, int accumulate) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_elem;
-         i += (long long)gridDim.x * blockDim.x) {
-        double s = accumulate ? (double)out[i] : 0.0;
-        for (long long c = 0; c < n_chunks; ++c) s += (double)partial[c * n_elem + i];
-        out[i] = (float)s;
+// Sums of the chunks' partial sums in FP64: a thread per element and eighth of the chunks, the eighths added in order.
+// One thread per element left the loads of its chunks one behind the other: 15,984 elements of 64 chunks 16.7 -> 8.3 us.
+constexpr int kReduceParts = 8;
+__global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, long long n_chunks,
+                                                             long long n_elem, float* __restrict__ out, int accumulate) {
+    __shared__ double s_part[kReduceParts][32];
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const long long per = (n_chunks + kReduceParts - 1) / kReduceParts;
+    const long long c0 = part * per, c1 = c0 + per < n_chunks ? c0 + per : n_chunks;
+    for (long long base = (long long)blockIdx.x * 32; base < n_elem; base += (long long)gridDim.x * 32) {
+        const long long i = base + lane;
+        double s = 0.0;
+        if (i < n_elem) {
+#pragma unroll 8
+            for (long long c = c0; c < c1; ++c) s += (double)partial[c * n_elem + i];
+        }
+        s_part[part][lane] = s;
+        __syncthreads();
+        if (part == 0 && i < n_elem) {
+            s = accumulate ? (double)out[i] : 0.0;
+#pragma unroll
+            for (int k = 0; k < kReduceParts; ++k) s += s_part[k][lane];
+            out[i] = (float)s;
+        }
+        __syncthreads();
     }
 }
 
@@ -764,7 +896,7 @@ cudaError_t launch_reduce_partials(const float* partial, long long n_chunks, lon
                                    int accumulate, cudaStream_t stream) {
     const long long n_elem = 6 * n_snk;
     if (n_elem == 0) return cudaSuccess;
-    const unsigned blocks = capped_blocks(n_elem, 256, 16);
+    const unsigned blocks = capped_blocks(n_elem, 32, 64);
     reduce_partials_kernel<<<blocks, 256, 0, stream>>>(partial, n_chunks, n_elem, out, accumulate); note_launches(1);
     return cudaGetLastError();
 }

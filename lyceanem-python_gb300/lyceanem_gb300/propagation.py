@@ -197,6 +197,14 @@ def pair_stage(src_pos, src_E, snk_pos, snk_nrm, *, beta, alpha=0.0, tris=None, 
         T = tri_t.shape[0]
         cs = ct = cb = None
         org, cell, dims = f32arr([0, 0, 0]), 1.0, i32arr([1, 1, 1])
+        # a warp drops the triangles outside its rays' beam: from about 1.3e8 pairs x triangles on, sinks in direction
+        # order from the first source gain more than the order costs (64 sources, 2,664 sinks, 1,024 triangles: 0.24
+        # against 0.16 + 0.03 ms).  Results do not depend on the order.
+        if snk_order is None and N * M * T >= 1 << 27:
+            snk_order = torch.empty(M, dtype=torch.int32, device=dev)
+            ws = _ws(lib.lyem_spatial_order_workspace(M), dev)
+            check(lib.lyem_direction_order_from(_p(tp), M, _p(sp), _p(snk_order), _p(ws), ws.numel(), _stream()),
+                  "direction_order")
     if sink_out is None:
         sink_out = torch.empty((M, 3), dtype=torch.complex64, device=dev)
         accumulate = False

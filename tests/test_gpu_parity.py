@@ -515,6 +515,32 @@ def test_spatial_order_is_the_stable_morton_sort(n):
     assert np.array_equal(P.spatial_order(pts).cpu().numpy(), np.argsort(key, kind="stable"))
 
 
+@pytest.mark.parametrize("n_src,n_snk,n_tris", [(1, 31, 31), (2, 33, 33), (3, 129, 127), (2, 160, 129), (40, 97, 300)])
+@pytest.mark.parametrize("cull", [True, False])
+@pytest.mark.parametrize("spread", ["beam", "around", "surface"])
+def test_brute_force_beam_culling(n_src, n_snk, n_tris, cull, spread):
+    """The per-warp culling of the brute-force kernel at the edges of its 32-triangle steps and tiles: sinks in one
+    direction (a beam), all around the sources (no beam), and sources and sinks on the triangles themselves, some of
+    them coincident; masks equal to the oracle's."""
+    P = _P()
+    rng = np.random.default_rng(n_src + n_snk + n_tris)
+    src, snk, snk_n, v, f, E = random_scene(n_src * 31 + n_snk, n_src=n_src, n_snk=n_snk, n_tris=n_tris)
+    if spread == "beam":
+        snk = (np.array([3.0, 1.0, 0.5]) + rng.uniform(-0.6, 0.6, (n_snk, 3))).astype(np.float32)
+    elif spread == "surface":
+        cen = v[f].mean(1)
+        src = cen[rng.integers(0, n_tris, n_src)].astype(np.float32)
+        snk = cen[rng.integers(0, n_tris, n_snk)].astype(np.float32)
+    tris = P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f))
+    kw = dict(self_to_self=True, cull=cull, eps=1e-6 if cull else 1e-7)
+    om = O.mask_brute(src, snk, O.pack_triangles(v, f), **kw)
+    r = P.pair_stage(src, E, snk, snk_n, beta=30.0, tris=tris, want_mask=True, **kw)
+    assert np.array_equal(r.mask().cpu().numpy(), om)
+    ro = P.pair_stage(src, E, snk, snk_n, beta=30.0, tris=tris, want_mask=True, snk_order=P.spatial_order(snk), **kw)
+    assert torch.equal(ro.mask_bits, r.mask_bits)
+    _no_device_errors()
+
+
 def test_stage_buffer_checks():
     """Caller buffers of the wrong type or length are refused before any launch (the kernels index them
     without bounds checks)."""

@@ -19,7 +19,7 @@
 // subnormal); the epilogue divides it out exactly.
 //
 // Kernel: persistent, one CTA of 192 threads per SM; a tile is 128 sinks x 256
-// beams of one component.  Warp 0 issues TMA loads of [A hi | A lo | B hi | B lo]
+// beams (fewer for small sweeps) of one component.  Warp 0 issues TMA loads of [A hi | A lo | B hi | B lo]
 // k-blocks into a ring of shared-memory stages; warp 1 owns the 512 TMEM
 // columns and issues the MMAs (M 128, N 256, K 16 per instruction) from one
 // thread; warps 2-5 (one TMEM lane quadrant each) run the epilogue.  A tile
@@ -44,16 +44,16 @@ namespace lyem {
 namespace {
 
 constexpr int kBM = 128;         // sinks per tile: TMEM lanes
-constexpr int kBN = 256;         // beams per tile: columns of one accumulator
 constexpr int kTcThreads = 192;  // warp 0 TMA, warp 1 MMA + TMEM owner, warps 2-5 epilogue
-constexpr int kTmemCols = 512;   // two accumulators of kBN FP32 columns
+constexpr int kTmemCols = 512;   // two accumulators of up to 256 FP32 columns
 
-template <int BK>
+// BN: beams per tile, the columns of one accumulator (tile_beams); the stages fill the same 192 KB.
+template <int BK, int BN>
 struct TcCfg {
     static constexpr int kRowBytes = BK * 2;                      // one swizzled operand row
-    static constexpr int kStages = BK == 64 ? 2 : 4;
+    static constexpr int kStages = (BN == 256 ? 4 : BN == 128 ? 6 : 8) / (BK / 32);
     static constexpr int kABytes = kBM * BK * 2;                  // one network tile (hi or lo)
-    static constexpr int kBBytes = kBN * BK * 2;                  // one weight tile (hi or lo)
+    static constexpr int kBBytes = BN * BK * 2;                  // one weight tile (hi or lo)
     static constexpr int kStageBytes = 2 * kABytes + 2 * kBBytes;
     static constexpr int kKSteps = BK / 16;                       // MMAs per operand pair and stage
     static constexpr int kBarriers = 2 * kStages + 6;
@@ -75,11 +75,11 @@ struct TcParams {
 // so each SM requests 2/3 of the operand bytes of a stage, and a stage is
 // refilled only after both CTAs' MMAs have read it (its empty barrier counts an
 // arrival from each).
-template <int BK, bool BF16, bool MC>
+template <int BK, int BN, bool BF16, bool MC>
 __global__ void __launch_bounds__(kTcThreads, 1)
     sweep_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const TcParams p) {
-    using C = TcCfg<BK>;
+    using C = TcCfg<BK, BN>;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // swizzled tiles need 1024-byte alignment
@@ -178,13 +178,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         tc::tma_load_3d(st + C::kABytes, &tmA, x, mt * kBM, pa + 1, fb);
                         if (MC) {  // this CTA's half of the weight rows, into both CTAs
                             const uint32_t half = (uint32_t)rank * (C::kBBytes / 2);
-                            const int y = kt * kBN + rank * (kBN / 2);
+                            const int y = kt * BN + rank * (BN / 2);
                             tc::tma_load_3d_mc(st + 2 * C::kABytes + half, &tmB, x, y, 2 * q, fb, 0x3);
                             tc::tma_load_3d_mc(st + 2 * C::kABytes + C::kBBytes + half, &tmB, x, y, 2 * q + 1, fb,
                                                0x3);
                         } else {
-                            tc::tma_load_3d(st + 2 * C::kABytes, &tmB, x, kt * kBN, 2 * q, fb);
-                            tc::tma_load_3d(st + 2 * C::kABytes + C::kBBytes, &tmB, x, kt * kBN, 2 * q + 1, fb);
+                            tc::tma_load_3d(st + 2 * C::kABytes, &tmB, x, kt * BN, 2 * q, fb);
+                            tc::tma_load_3d(st + 2 * C::kABytes + C::kBBytes, &tmB, x, kt * BN, 2 * q + 1, fb);
                         }
                         issued[s] = true;
                         last_par[s] = ph;
@@ -200,13 +200,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
     } else if (warp == 1) {
         if (lane == 0) {  // MMA issuer
-            constexpr uint32_t idesc = tc::idesc_f16(BF16, kBM, kBN);
+            constexpr uint32_t idesc = tc::idesc_f16(BF16, kBM, BN);
             int s = 0, it = 0;
             uint32_t ph = 0;
             bool ok = true;
             for (int t = first; ok && t < tiles; t += step, ++it) {
                 for (int q = 0; ok && q < 3; ++q) {
-                    const uint32_t acc = tmem + (q == 0 ? 0u : (uint32_t)kBN);
+                    const uint32_t acc = tmem + (q == 0 ? 0u : (uint32_t)BN);
                     bool w = true;
                     if (q == 0 && it > 0) w = wait(bar(ACC0_EMPTY), (uint32_t)(it - 1) & 1u);
                     if (q == 1 && it > 0) w = wait(bar(ACC1_EMPTY), (uint32_t)(it - 1) & 1u);
@@ -276,14 +276,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             float* out = p.out + (size_t)c * p.n_beams * p.ldc * 2;
             auto write_part = [&](uint32_t col0, int part) {
 #pragma unroll 1
-                for (int j = 0; j < kBN / 32; ++j) {
+                for (int j = 0; j < BN / 32; ++j) {
                     float v[32];
                     __syncwarp();  // tcgen05.ld is a .sync.aligned warp instruction
                     tc::tmem_ld32(tmem + lane_off + col0 + (uint32_t)j * 32u, v);
                     if (m < p.n_snk) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
-                            const long long k = (long long)kt * kBN + j * 32 + i;
+                            const long long k = (long long)kt * BN + j * 32 + i;
                             if (k < p.n_beams) out[(k * p.ldc + m) * 2 + part] = v[i] * inv;
                         }
                     }
@@ -293,9 +293,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             if (!wait_warp(bar(MID_FULL), (uint32_t)it & 1u)) break;
             tc::fence_after();
 #pragma unroll 1
-            for (int j = 0; j < kBN / 32; ++j) {
+            for (int j = 0; j < BN / 32; ++j) {
                 float a[32], b[32];
-                const uint32_t ta = tmem + lane_off + (uint32_t)j * 32u, tb = ta + (uint32_t)kBN;
+                const uint32_t ta = tmem + lane_off + (uint32_t)j * 32u, tb = ta + (uint32_t)BN;
                 __syncwarp();
                 tc::tmem_ld32x2(ta, tb, a, b);
 #pragma unroll
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             signal(bar(ACC0_EMPTY));
             if (!wait_warp(bar(ACC_FULL), (uint32_t)it & 1u)) break;
             tc::fence_after();
-            write_part((uint32_t)kBN, 1);
+            write_part((uint32_t)BN, 1);
             signal(bar(ACC1_EMPTY));
         }
     }
@@ -364,11 +364,11 @@ bool make_map(CUtensorMap* m, const void* base, bool bf16, int k, int rows, int 
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BK, bool BF16, bool MC>
+template <int BK, int BN, bool BF16, bool MC>
 cudaError_t launch_tc(const CUtensorMap& a, const CUtensorMap& b, const TcParams& p, cudaStream_t stream,
                       bool* launched) {
-    using C = TcCfg<BK>;
-    auto kern = sweep_tc_kernel<BK, BF16, MC>;
+    using C = TcCfg<BK, BN>;
+    auto kern = sweep_tc_kernel<BK, BN, BF16, MC>;
     *launched = false;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
     if (e != cudaSuccess) return e;
@@ -405,6 +405,37 @@ cudaError_t launch_tc(const CUtensorMap& a, const CUtensorMap& b, const TcParams
     return cudaGetLastError();
 }
 
+template <int BN>
+cudaError_t launch_single(int bk, bool bf16, const CUtensorMap& a, const CUtensorMap& b, const TcParams& p,
+                          cudaStream_t stream) {
+    bool done = false;
+    if (bk == 64)
+        return bf16 ? launch_tc<64, BN, true, false>(a, b, p, stream, &done)
+                    : launch_tc<64, BN, false, false>(a, b, p, stream, &done);
+    return bf16 ? launch_tc<32, BN, true, false>(a, b, p, stream, &done)
+                : launch_tc<32, BN, false, false>(a, b, p, stream, &done);
+}
+
+// Beams per tile.  256 keeps the tensor pipe fullest; where its tiles leave SMs idle or are mostly padding, narrower ones
+// shorten the launch: the width of least cost, waves of tiles times (width + 96), 96 standing for the share of a tile's time
+// that does not shrink with it (network rows, pipeline fill).  Whole sweeps with 256 / 128 / 64: 961 sources, 2,701 sinks, 181 beams
+// 142 / 121 / 145 us, 64 beams 129 / 108 / 102, 400 beams 154 / 176 / 220; 4,096 x 65,341, 100 beams 2.10 / 1.73 /
+// 2.83 ms, 256 beams 2.72 / 2.98 / 5.48.
+int tile_beams(long long row_tiles, long long n_beams) {
+    const long long sms = device_sm_count();
+    int best = 256;
+    long long cost = 0;
+    for (int bn = 256; bn >= 64; bn /= 2) {
+        const long long waves = (3 * row_tiles * ((n_beams + bn - 1) / bn) + sms - 1) / sms;
+        const long long c = waves * (bn + 96);
+        if (bn == 256 || c < cost) {
+            best = bn;
+            cost = c;
+        }
+    }
+    return best;
+}
+
 }  // namespace
 
 int sweep_tc_k_tile = 32;
@@ -416,17 +447,18 @@ int launch_sweep_tc(const void* network, const void* weights, int64_t n_src, int
     const long long kpad = (n_src + 7) / 8 * 8;
     const unsigned char* na = static_cast<const unsigned char*>(network);
     const unsigned char* wb = static_cast<const unsigned char*>(weights);
-    CUtensorMap ma, mb, mb_half;
+    const int n_mt = (int)((n_snk + kBM - 1) / kBM);
+    const int bn = sweep_tc_multicast ? 256 : tile_beams(n_mt, n_beams);
+    CUtensorMap ma, mb;
     if (!make_map(&ma, na + kSweepHeaderBytes, bf16, (int)n_src, (int)n_snk, 18, kpad, ld, bk, kBM) ||
-        !make_map(&mb, wb + kSweepHeaderBytes, bf16, (int)n_src, (int)n_beams, 6, kpad, n_beams, bk, kBN) ||
-        !make_map(&mb_half, wb + kSweepHeaderBytes, bf16, (int)n_src, (int)n_beams, 6, kpad, n_beams, bk, kBN / 2))
+        !make_map(&mb, wb + kSweepHeaderBytes, bf16, (int)n_src, (int)n_beams, 6, kpad, n_beams, bk, bn))
         return LYEM_ERR_CUDA;
     TcParams p;
     p.n_src = (int)n_src;
     p.n_snk = (int)n_snk;
     p.n_beams = (int)n_beams;
-    p.n_mt = (int)((n_snk + kBM - 1) / kBM);
-    p.n_kt = (int)((n_beams + kBN - 1) / kBN);
+    p.n_mt = n_mt;
+    p.n_kt = (int)((n_beams + bn - 1) / bn);
     p.n_kb = (int)((n_src + bk - 1) / bk);
     p.ldc = ldc;
     p.out = out;
@@ -437,21 +469,20 @@ int launch_sweep_tc(const void* network, const void* weights, int64_t n_src, int
     cudaError_t e = cudaSuccess;
     bool done = false;
     if (sweep_tc_multicast) {  // clusters of two sharing the weight tile; the single-CTA kernel if none fit
+        CUtensorMap mb_half;
+        if (!make_map(&mb_half, wb + kSweepHeaderBytes, bf16, (int)n_src, (int)n_beams, 6, kpad, n_beams, bk, bn / 2))
+            return LYEM_ERR_CUDA;
         if (bk == 64)
-            e = bf16 ? launch_tc<64, true, true>(ma, mb_half, p, stream, &done)
-                     : launch_tc<64, false, true>(ma, mb_half, p, stream, &done);
+            e = bf16 ? launch_tc<64, 256, true, true>(ma, mb_half, p, stream, &done)
+                     : launch_tc<64, 256, false, true>(ma, mb_half, p, stream, &done);
         else
-            e = bf16 ? launch_tc<32, true, true>(ma, mb_half, p, stream, &done)
-                     : launch_tc<32, false, true>(ma, mb_half, p, stream, &done);
+            e = bf16 ? launch_tc<32, 256, true, true>(ma, mb_half, p, stream, &done)
+                     : launch_tc<32, 256, false, true>(ma, mb_half, p, stream, &done);
     }
-    if (e == cudaSuccess && !done) {
-        if (bk == 64)
-            e = bf16 ? launch_tc<64, true, false>(ma, mb, p, stream, &done)
-                     : launch_tc<64, false, false>(ma, mb, p, stream, &done);
-        else
-            e = bf16 ? launch_tc<32, true, false>(ma, mb, p, stream, &done)
-                     : launch_tc<32, false, false>(ma, mb, p, stream, &done);
-    }
+    if (e == cudaSuccess && !done)
+        e = bn == 256 ? launch_single<256>(bk, bf16, ma, mb, p, stream)
+            : bn == 128 ? launch_single<128>(bk, bf16, ma, mb, p, stream)
+                        : launch_single<64>(bk, bf16, ma, mb, p, stream);
     if (e != cudaSuccess) {
         record_cuda_error(e);
         return LYEM_ERR_CUDA;

@@ -776,6 +776,28 @@ def test_beam_sweep_fp16_scaling(scale):
         assert err < SWEEP_TOL, (mode, scale, err)
 
 
+@pytest.mark.parametrize("k_tile", [32, 64])
+@pytest.mark.parametrize("n_src,n_snk,n_beams", [(33, 129, 63), (40, 129, 65), (24, 6400, 129), (30, 6401, 257),
+                                                 (17, 12000, 64)])
+def test_beam_sweep_tile_widths(k_tile, n_src, n_snk, n_beams):
+    """Sweeps whose rule picks 64, 128 and 256 beams a tile, with ragged rows and columns, against FP64."""
+    from lyceanem_gb300 import beam_sweep as BS
+    gen = torch.Generator("cuda").manual_seed(n_snk + n_beams)
+    G = torch.randn((n_src, n_snk, 3), dtype=torch.complex64, device="cuda", generator=gen)
+    W = torch.randn((n_beams, n_src), dtype=torch.complex64, device="cuda", generator=gen)
+    BS.set_k_tile(k_tile)
+    try:
+        sw = BS.BeamSweep(G, "bf16x3g")
+        E = sw.fields(sw.run(W))
+    finally:
+        BS.set_k_tile(32)
+    ref = torch.einsum("nmc,kn->mkc", G.to(torch.complex128), W.to(torch.complex128))
+    # the dropped lo*lo terms and the halves' rounding: 2^-16 of |G||W| summed over the sources
+    bound = torch.einsum("nmc,kn->mkc", G.abs().double(), W.abs().double()) * (3 * 2.0 ** -16)
+    assert ((E - ref).abs() <= bound).all()
+    _no_device_errors()
+
+
 def test_beam_sweep_repeat_and_reuse():
     """Two runs of one prepared sweep give identical results (the kernel writes every output once, from
     a fixed accumulation order), and a second weight set reuses the operand."""

@@ -251,13 +251,16 @@ __device__ __forceinline__ void pair_freqs(const BatchParams& P, float ox, float
     const float sc = -0.15915494309189535f * nd * mag;  // -(1/2pi) (n.d) exp(-alpha r)/r
     float rh, rl;
     ff_length(ox, oy, oz, ex, ey, ez, rh, rl);
-    float sn, cs;
-    sincosf(ff_phase(b0.x, b0.y, rh, rl), &sn, &cs);
+    // both phases with what their FP32 rounding drops: the rotation below multiplies that of the step up to FG - 1 times
+    float sn, cs, rem;
+    const float ph = ff_phase_parts(b0.x, b0.y, rh, rl, rem);
+    sincos_parts(ph, rem, &sn, &cs);
     float cre = sc * cs, cim = -sc * sn;  // sc exp(-j beta_f0 r)
     float zre = 1.f, zim = 0.f;
     if (FG > 1) {
         float zs, zc;
-        sincosf(ff_phase(P.dbeta_ff.x, P.dbeta_ff.y, rh, rl), &zs, &zc);
+        const float dph = ff_phase_parts(P.dbeta_ff.x, P.dbeta_ff.y, rh, rl, rem);
+        sincos_parts(dph, rem, &zs, &zc);
         zre = zc;
         zim = -zs;
     }

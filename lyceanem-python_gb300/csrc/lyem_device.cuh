@@ -404,6 +404,31 @@ __device__ __forceinline__ float ff_phase(float bh, float bl, float rh, float rl
     return __fadd_rn(x, lo);
 }
 
+// The same phase with its small terms (the products' low parts and k*kC2) kept apart: x + rem is it to about
+// 1e-8 rad for |phase| up to 2^20, with x its FP32 rounding.
+__device__ __forceinline__ float ff_phase_parts(float bh, float bl, float rh, float rl, float& rem) {
+    const float kC1 = 6.28318548202514648f;
+    const float kC2 = -1.74845553146951715e-7f;
+    const float kInv = 0.159154936671257019f;
+    const float p = __fmul_rn(bh, rh);
+    const float pe = __fmaf_rn(bh, rh, -p);
+    const float lo = __fadd_rn(pe, __fmaf_rn(bh, rl, __fmul_rn(bl, rh)));
+    const float k = rintf(__fmul_rn(p, kInv));
+    const float x0 = __fmaf_rn(-k, kC1, p);  // exact, as in ff_phase
+    const float t = __fmaf_rn(-k, kC2, lo);
+    float x;
+    two_sum(x0, t, x, rem);
+    return x;
+}
+
+// cos and sin of x + rem for a rem of the size of x's rounding.
+__device__ __forceinline__ void sincos_parts(float x, float rem, float* s, float* c) {
+    float s0, c0;
+    sincosf(x, &s0, &c0);
+    *s = __fmaf_rn(rem, c0, s0);
+    *c = __fmaf_rn(-rem, s0, c0);
+}
+
 // Bounded wait on an mbarrier phase.  Returns false if the deadline (in SM
 // clock cycles) passes first; the caller then reports LYEM_ERR_TIMEOUT.
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar_addr, uint32_t parity, long long max_cycles) {

@@ -34,14 +34,22 @@ C0 = 299792458.0
 
 # (frequencies per thread, sources per visibility item, blocks per SM).  Blocks per
 # SM 3, 4, 6 or 8 select kernel variants whose registers are capped for that
-# occupancy; 0 runs the uncapped variant with as many blocks as fit.  On the
-# 64-scene batch with one 0.5 m cell (4.0e9 ray pairs, 9.9e11 ray-triangle tests) one launch took
-# 5.41 s at (4, 64, 4) and 4.49 / 5.36 / 4.71 s at (2 / 1 / 4, 64, 8): the
-# visibility phase dominates and gains from the extra resident warps more
-# than the field phase loses to spilling.
-CANDIDATES = [(2, 64, 8), (2, 64, 6), (1, 64, 8), (4, 64, 8), (2, 32, 8), (4, 64, 4), (4, 32, 3), (8, 32, 3),
-              (4, 32, 0)]
-DEFAULT = (2, 64, 8)
+# occupancy; 0 runs the uncapped variant with as many blocks as fit.
+CANDIDATES = [(2, 64, 8), (2, 64, 6), (2, 32, 6), (1, 32, 8), (2, 32, 8), (4, 64, 4), (4, 32, 4), (4, 32, 3), (8, 32, 3)]
+
+
+def default_config(n_freq, pairs, uniform):
+    """Configuration of a batch that is not tuned.  Few frequencies: one per thread (the pair set-up is not shared, so
+    threads go to sinks), and the most warps for the walks.  More: four per thread, which share the set-up, unless the
+    walks dominate (200 million ray pairs and more), which want the warps.  Milliseconds at (2, 64, 8) / (1, 32, 8) /
+    (2, 32, 6) / (4, 32, 4): 8 scenes, 1e8 pairs, 1 frequency 36.9 / 29.4 / 32.3 / 34.3, 4 frequencies 41.5 / 31.7 /
+    34.3 / 38.0, 16 frequencies 59.3 / 56.4 / 47.5 / 45.9, 64 frequencies 131 / 159 / 112 / 81; 24 scenes, 6e8 pairs, 16
+    frequencies 190 / 196 / 183 / 196; 3 small scenes, 7 frequencies 8.5 / 8.3 / 6.7 / 4.4."""
+    if n_freq <= 4 or not uniform:
+        return (1, 32, 8)
+    if n_freq < 32 and pairs >= 2e8:
+        return (2, 32, 6)
+    return (4, 32, 4)
 
 
 def stratified_subset(scenes, n_sinks, every=4):
@@ -198,7 +206,7 @@ class BatchedScattering:
     # ------------------------------------------------------------ configuration
 
     def _default(self):
-        return DEFAULT if self.uniform else (1, DEFAULT[1], DEFAULT[2])
+        return default_config(self.n_freq, self.pairs(), self.uniform)
 
     def _cfg(self, c):
         cfg = BatchConfig()

@@ -90,6 +90,9 @@ struct BatchParams {
     const DevScene* scenes;
     const int4* items;  // (kind, scene, a, b)
     int n_items;
+    int n_vis;      // V items, the first of the list
+    int split;      // parts of a V item (a power of two up to 32): queue positions 0 .. n_vis * split - 1 are its parts
+    int turn_all;   // the scatter -> sink items are turned as well
     int n_scenes;
     unsigned int* head;  // queue position
     unsigned int* done;  // [n_scenes][kKinds] finished items
@@ -132,9 +135,10 @@ __device__ bool wait_count(const unsigned* ctr, unsigned target) {
 __device__ bool wait_deps(const BatchParams& P, int kind, int scene) {
     const DevScene& S = P.scenes[scene];
     const unsigned* d = P.done + (long long)scene * kKinds;
-    if (kind == kFieldW) return wait_count(d + kVisScat, (unsigned)S.expect[kVisScat]);
-    bool ok = wait_count(d + kVisDirect, (unsigned)S.expect[kVisDirect]);
-    ok = ok && wait_count(d + kVisBounce, (unsigned)S.expect[kVisBounce]);
+    const unsigned parts = (unsigned)P.split;
+    if (kind == kFieldW) return wait_count(d + kVisScat, (unsigned)S.expect[kVisScat] * parts);
+    bool ok = wait_count(d + kVisDirect, (unsigned)S.expect[kVisDirect] * parts);
+    ok = ok && wait_count(d + kVisBounce, (unsigned)S.expect[kVisBounce] * parts);
     ok = ok && wait_count(d + kFieldW, (unsigned)S.expect[kFieldW]);
     return ok;
 }
@@ -151,7 +155,7 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 // the caller) rather than held in registers through the walk.
 template <bool CULL>
 __device__ void vis_item(const BatchParams& P, const DevScene& S, const GridView& G, int scene, int stage,
-                         long long n0, long long m0) {
+                         long long n0, long long m0, int i0, int i1) {
     const int lane = threadIdx.x & 31;
     const float* spos = stage == kVisBounce ? S.scat_pos : S.src_pos;
     const long long ns = stage == kVisBounce ? S.n_scat : S.n_src;
@@ -177,9 +181,11 @@ __device__ void vis_item(const BatchParams& P, const DevScene& S, const GridView
     // The element stages turn the warp round: the lanes are 32 of the chunk's sources (an array's elements) and the
     // warp walks to one sink after the other, so its rays cross the same cells (as grid_transposed_kernel does; 8 scenes
     // of up to 3,969 elements, 16 frequencies: 64.0 -> 59.3 ms at (2, 64, 8), 57.1 -> 46.6 at (2, 32, 6)).
-    const bool turned = stage != kVisBounce;
+    // Scatter points as sources are turned for few sinks, which lie too far apart to share a walk (the rule of
+    // propagation.scatter_schedule), and where items are split; a part of an item holds its sinks i0 .. i1 - 1.
+    const bool turned = stage != kVisBounce || P.turn_all;
     for (int g = 0; g < nsrc; g += 32) {
-        const int iters = turned ? kWarpSinks : min(32, nsrc - g);
+        const int first = turned ? i0 : 0, last = turned ? i1 : min(32, nsrc - g);
         const bool n_ok = g + lane < nsrc;
         unsigned int word = 0;
         float lx = ex, ly = ey, lz = ez;  // the lane's end point: its sink, or its source where turned
@@ -187,7 +193,7 @@ __device__ void vis_item(const BatchParams& P, const DevScene& S, const GridView
             const float* so = spos + 3 * (n0 + g + (n_ok ? lane : 0));
             lx = __ldg(so); ly = __ldg(so + 1); lz = __ldg(so + 2);
         }
-        for (int i = 0; i < iters; ++i) {
+        for (int i = first; i < last; ++i) {
             const long long n = n0 + g + (turned ? (n_ok ? lane : 0) : i);
             const long long k = turned ? m0 + i : ms;
             if (turned && k >= nk) break;  // the same in every lane
@@ -221,8 +227,10 @@ __device__ void vis_item(const BatchParams& P, const DevScene& S, const GridView
                 word |= 1u << i;
             }
         }
-        if (ok) S.mask[stage][ms * S.mask_words[stage] + ((n0 + g) >> 5)] = word;
-        vis += __popc(ok ? word : 0u);
+        if (ok && (!turned || (lane >= i0 && lane < i1))) {
+            S.mask[stage][ms * S.mask_words[stage] + ((n0 + g) >> 5)] = word;
+            vis += __popc(word);
+        }
     }
     if (P.counters) {
         const unsigned long long v = warp_sum(vis);
@@ -422,9 +430,16 @@ __global__ void __launch_bounds__(kBT, MINB) batch_kernel(const BatchParams P) {
     unsigned nxt = 0;
     if (lane == 0) nxt = atomicAdd(P.head, 1u);
     while (true) {
-        int kind = -1, scene = 0, a = 0, b = 0, run = 1;
+        int kind = -1, scene = 0, a = 0, b = 0, run = 1, part = 0;
         if (lane == 0) {
-            const unsigned i = nxt;
+            unsigned i = nxt;
+            const unsigned parts = (unsigned)P.n_vis * (unsigned)P.split;
+            if (i < parts) {
+                part = (int)(i & (unsigned)(P.split - 1));
+                i /= (unsigned)P.split;
+            } else {
+                i -= parts - (unsigned)P.n_vis;
+            }
             if (i < (unsigned)P.n_items) {
                 const int4 it = P.items[i];
                 kind = it.x;
@@ -444,12 +459,14 @@ __global__ void __launch_bounds__(kBT, MINB) batch_kernel(const BatchParams P) {
         a = __shfl_sync(full, a, 0);
         b = __shfl_sync(full, b, 0);
         run = __shfl_sync(full, run, 0);
+        part = __shfl_sync(full, part, 0);
         __syncwarp();  // s_grid[wid] is visible to the warp
         if (kind < 0) break;
         if (run) {
             const DevScene& S = P.scenes[scene];
             if (kind < kFieldW)
-                vis_item<CULL>(P, S, s_grid[wid], scene, kind, (long long)a, (long long)b);
+                vis_item<CULL>(P, S, s_grid[wid], scene, kind, (long long)a, (long long)b,
+                               part * (kWarpSinks / P.split), (part + 1) * (kWarpSinks / P.split));
             else
                 for (int t = 0; t < b; ++t)  // b consecutive 32-slot chunks
                     field_item<FG>(P, S, scene, kind, (long long)a + t, sacc);
@@ -594,7 +611,7 @@ void beta_tables(const double* beta, int n, std::vector<float2>& ff, std::vector
 }
 
 template <bool CULL, int FG, int MINB>
-cudaError_t launch_batch_t(const BatchParams& P, int blocks_per_sm, cudaStream_t stream, int* blocks_out) {
+cudaError_t launch_batch_t(BatchParams P, int blocks_per_sm, cudaStream_t stream, int* blocks_out) {
     auto kern = batch_kernel<CULL, FG, MINB>;
     const size_t smem = sizeof(float) * 6 * FG * kBT;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -605,7 +622,15 @@ cudaError_t launch_batch_t(const BatchParams& P, int blocks_per_sm, cudaStream_t
     const int per_sm = blocks_per_sm > 0 ? std::min(blocks_per_sm, std::max(fit, 1)) : std::max(fit, 1);
     const int sms = device_sm_count();
     if (sms <= 0) return cudaErrorInvalidDevice;
-    const int blocks = std::max(1, std::min(per_sm * sms, P.n_items));
+    // A V item is 32 or 64 walks (or twice that, turned) one behind the other: the items are split into parts until there
+    // are four for every resident warp.  At (2, 64, 8): 2 scenes of up to 64 elements, 500 sinks, 1 frequency 3.12 -> 1.52
+    // ms; 4 of up to 986, 673 sinks, 1 frequency 6.54 -> 2.49; 2 of up to 300, 4,000 sinks, 3 frequencies 24.4 -> 16.7; 8 of
+    // up to 3,969, 4,000 sinks, 16 frequencies 57.2 -> 52.5 (one part a warp 55.9, 16 parts 50.8).
+    const long long want = (long long)per_sm * sms * (kBT / 32) * 4;
+    P.split = 1;
+    while (P.split < kWarpSinks && (long long)P.n_vis * P.split < want) P.split *= 2;
+    P.turn_all = P.split > 1 || P.n_snk <= 2048;
+    const int blocks = (int)std::max(1LL, std::min<long long>((long long)per_sm * sms, P.n_items + (long long)P.n_vis * (P.split - 1)));
     kern<<<blocks, kBT, smem, stream>>>(P);
     note_launches(1);
     if (blocks_out) *blocks_out = blocks;
@@ -750,6 +775,8 @@ LYEM_API int lyem_batch_launch(const lyem_batch_scene* scenes, int32_t n_scenes,
     P.scenes = reinterpret_cast<const DevScene*>(base + pl.off_scenes);
     P.items = reinterpret_cast<const int4*>(base + pl.off_items);
     P.n_items = (int)pl.items.size();
+    P.n_vis = 0;
+    while (P.n_vis < P.n_items && pl.items[P.n_vis].x < kFieldW) ++P.n_vis;
     P.n_scenes = n_scenes;
     P.head = reinterpret_cast<unsigned int*>(base + pl.off_ctrl);
     P.done = P.head + 1;

@@ -211,3 +211,29 @@ def test_density_cells_same_field(small, tmp_path, monkeypatch):
     cached = again.autotune(candidates=[(2, 64, 0), (4, 32, 4)], cell_scales=[0.8, 1.2])
     assert list(cached) == [best] and again.cell_scale == best[3] and again.grid_cells() == bs.grid_cells()
     assert P.device_errors() == (0, 0)
+
+
+@pytest.mark.parametrize("copies", [1, 8, 30, 60])
+@pytest.mark.parametrize("n_snk", [250, 2100])
+def test_split_visibility_items(copies, n_snk):
+    """Launches whose visibility items are split into 32, 4, 2 and no parts (the copies of one scene set how many
+    items there are), with few sinks (every item turned) and more (scatter items in lockstep where not split): every
+    copy gives the counts and the field of the per-scene pair stages."""
+    B, P, SC = _mods()
+    rng = np.random.default_rng(7)
+    sc = _scene(SC, rng, 8, 200, 8, 150, B.C0 / 27e9)
+    snk, snk_n = SC.fibonacci_sinks(50.0, n_snk)
+    b = B.BatchedScattering([sc] * copies, snk, snk_n, [27e9], cell_scale=1.5, config=(4, 32, 3))
+    field = b.run().cpu().numpy()
+    counts = b.counters.cpu().numpy()
+    beta = float(B.betas_of([27e9])[0])
+    kw = dict(beta=beta, tris=P.pack_triangles(sc.verts, sc.faces))
+    cnt = torch.zeros((3, 2), dtype=torch.int64, device="cuda")
+    e_p = P.pair_stage(sc.src, sc.E, sc.scat, sc.scat_n, counters=cnt[0], **kw).sink
+    out = P.pair_stage(sc.src, sc.E, snk, snk_n, counters=cnt[1], **kw).sink
+    P.pair_stage(sc.scat, e_p, snk, snk_n, src_W=e_p, sink_out=out, accumulate=True, counters=cnt[2], **kw)
+    assert (counts[:, :3] == cnt[:, 0].cpu().numpy()).all()
+    for s in range(copies):
+        assert rel_err(field[s, 0], out.cpu().numpy()) < 2e-6  # FP32 sums of up to 150 terms in two orders
+    st, flags = P.device_errors()
+    assert st == 0 and flags == 0

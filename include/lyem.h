@@ -61,7 +61,7 @@ LYEM_API uint64_t lyem_kernel_launches(void);
  * FMA lane-operations per second, the denominator of the visibility roofline. */
 LYEM_API int lyem_fp32_fma_probe(int64_t iterations, double *fma_per_second, void *stream);
 /* Synchronises `stream`, then reads and clears the library's device error word
- * (bit 0: a bounded wait expired; bit 1: an index check failed).  Returns
+ * (bit 0: a bounded wait expired; the other bits are reserved).  Returns
  * LYEM_ERR_TIMEOUT if bit 0 was set. */
 LYEM_API int lyem_device_errors(void *stream, uint32_t *flags_out);
 

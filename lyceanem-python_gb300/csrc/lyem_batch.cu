@@ -215,7 +215,7 @@ __device__ void vis_item(const BatchParams& P, const DevScene& S, const GridView
                                 break;
                             }
                         }
-                        if (hit || !walk_step(G, w, P.err)) break;
+                        if (hit || !walk_step(G, w)) break;
                     }
                     seen = !hit;
                 }

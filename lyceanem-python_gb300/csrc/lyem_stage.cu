@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(kThreads, MODE == kLockstep10 ? 10 : (MODE == 
                             if (walk_test<CULL>(p, w)) { hit = true; break; }
                         }
                         if (hit) break;
-                        const int st = walk_step_until(p, w, near, &g_device_error);
+                        const int st = walk_step_until(p, w, near);
                         if (st != 1) {
                             far = st == 2;
                             break;
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kThreads, MODE == kLockstep10 ? 10 : (MODE == 
                             ++tests;
                             if (walk_test<CULL>(p, w)) { hit = true; break; }
                         }
-                        if (hit || !walk_step(p, w, &g_device_error)) break;
+                        if (hit || !walk_step(p, w)) break;
                     }
                 }
                 if (hit) atomicOr(&s_blk[warp][owner], 1ull << s);
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(kThreads, MODE == kLockstep10 ? 10 : (MODE == 
                     if (COUNT) ++tests;
                     if (walk_test<CULL>(p, w)) { hit = true; break; }
                 }
-                if (hit || !walk_step(p, w, &g_device_error)) break;
+                if (hit || !walk_step(p, w)) break;
             }
             if (hit) blocked |= 1ull << s;
         }
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(kThreads, MODE == kLockstep10 ? 10 : (MODE == 
                         break;
                     }
                 }
-                if (has && !walk_step(p, w, &g_device_error)) has = false;
+                if (has && !walk_step(p, w)) has = false;
             }
         }
     }
@@ -747,7 +747,7 @@ __global__ void __launch_bounds__(kThreads, 16) grid_transposed_kernel(const Sta
                         if (COUNT) ++tests;
                         if (walk_test<CULL>(p, w)) { hit = true; break; }
                     }
-                    if (hit || !walk_step(p, w, &g_device_error)) break;
+                    if (hit || !walk_step(p, w)) break;
                 }
             }
             vis = !hit;

@@ -15,8 +15,8 @@ namespace lyem {
 struct Walk {
     float ox, oy, oz;
     Ray r;
-    float ix, iy, iz, t1;
-    int cx, cy, cz, q, q1, guard;
+    float ix, iy, iz;
+    int cx, cy, cz, q, q1;
 };
 
 // True when the segment certainly misses box [lo, hi]: slab test over the
@@ -79,7 +79,7 @@ template <class GP>
 __device__ __forceinline__ bool walk_setup(const GP& p, Walk& w) {
     const float ox = w.ox, oy = w.oy, oz = w.oz;
     float t0 = 0.f;
-    w.t1 = w.r.len;
+    float t1 = w.r.len;
     bool miss = false;
 #define LYEM_SLAB(D, O, G0, G1, INV)                       \
     if (D == 0.f) {                                        \
@@ -89,17 +89,16 @@ __device__ __forceinline__ bool walk_setup(const GP& p, Walk& w) {
         INV = 1.0f / D;                                    \
         float ta = (G0 - O) * INV, tb = (G1 - O) * INV;    \
         t0 = fmaxf(t0, fminf(ta, tb));                     \
-        w.t1 = fminf(w.t1, fmaxf(ta, tb));                 \
+        t1 = fminf(t1, fmaxf(ta, tb));                     \
     }
     LYEM_SLAB(w.r.dx, ox, p.g0[0], p.g1[0], w.ix)
     LYEM_SLAB(w.r.dy, oy, p.g0[1], p.g1[1], w.iy)
     LYEM_SLAB(w.r.dz, oz, p.g0[2], p.g1[2], w.iz)
 #undef LYEM_SLAB
-    if (miss || !(t0 <= w.t1)) return false;
+    if (miss || !(t0 <= t1)) return false;
     w.cx = min(max((int)floorf((ox + t0 * w.r.dx - p.g0[0]) * p.inv_cell), 0), p.dims[0] - 1);
     w.cy = min(max((int)floorf((oy + t0 * w.r.dy - p.g0[1]) * p.inv_cell), 0), p.dims[1] - 1);
     w.cz = min(max((int)floorf((oz + t0 * w.r.dz - p.g0[2]) * p.inv_cell), 0), p.dims[2] - 1);
-    w.guard = p.dims[0] + p.dims[1] + p.dims[2] + 2;
     walk_enter(p, w, (w.cz * p.dims[1] + w.cy) * p.dims[0] + w.cx);
     return true;
 }
@@ -184,7 +183,7 @@ template <class GP>
 __device__ __forceinline__ bool walk_setup_from(const GP& p, Walk& w, float from) {
     const float ox = w.ox, oy = w.oy, oz = w.oz;
     float t0 = from;
-    w.t1 = w.r.len;
+    float t1 = w.r.len;
     bool miss = false;
 #define LYEM_SLAB(D, O, G0, G1, INV)                       \
     if (D == 0.f) {                                        \
@@ -194,17 +193,16 @@ __device__ __forceinline__ bool walk_setup_from(const GP& p, Walk& w, float from
         INV = 1.0f / D;                                    \
         float ta = (G0 - O) * INV, tb = (G1 - O) * INV;    \
         t0 = fmaxf(t0, fminf(ta, tb));                     \
-        w.t1 = fminf(w.t1, fmaxf(ta, tb));                 \
+        t1 = fminf(t1, fmaxf(ta, tb));                     \
     }
     LYEM_SLAB(w.r.dx, ox, p.g0[0], p.g1[0], w.ix)
     LYEM_SLAB(w.r.dy, oy, p.g0[1], p.g1[1], w.iy)
     LYEM_SLAB(w.r.dz, oz, p.g0[2], p.g1[2], w.iz)
 #undef LYEM_SLAB
-    if (miss || !(t0 <= w.t1)) return false;
+    if (miss || !(t0 <= t1)) return false;
     w.cx = min(max((int)floorf((ox + t0 * w.r.dx - p.g0[0]) * p.inv_cell), 0), p.dims[0] - 1);
     w.cy = min(max((int)floorf((oy + t0 * w.r.dy - p.g0[1]) * p.inv_cell), 0), p.dims[1] - 1);
     w.cz = min(max((int)floorf((oz + t0 * w.r.dz - p.g0[2]) * p.inv_cell), 0), p.dims[2] - 1);
-    w.guard = p.dims[0] + p.dims[1] + p.dims[2] + 2;
     walk_enter(p, w, (w.cz * p.dims[1] + w.cy) * p.dims[0] + w.cx);
     return true;
 }
@@ -224,59 +222,42 @@ __device__ __forceinline__ void next_crossings(const GP& p, const Walk& w, float
     if (w.r.dz == 0.f) tz = kInf;
 }
 
-// Crosses the nearest cell boundary unless the crossing lies at or beyond
-// parameter `stop`: 0 = the segment or the grid ends there, 1 = the next cell
-// was entered, 2 = stopped before a crossing at or beyond `stop`.
+// Crosses the nearest cell boundary; false when the segment or the grid ends there.  Each step moves one cell index
+// one way only (the sign of that direction component), so a walk ends after dims[0] + dims[1] + dims[2] steps at most,
+// whatever its numbers; and it ends at the grid's own last cell, so no exit parameter is kept.  The three cases are
+// selects, not branches: the lanes of a warp cross different axes, and a branch each is run one after the other.
+// (With a step counter, an exit parameter and branches, 5,000 scatter points: 42.96 against 41.2 ms to 65,341 sinks,
+// 9.17 against 8.6 ms to 16,471 sinks in numba's test.)
 template <class GP>
-__device__ __forceinline__ int walk_step_until(const GP& p, Walk& w, float stop, unsigned int* err) {
+__device__ __forceinline__ bool walk_cross(const GP& p, Walk& w, float tx, float ty, float tz, float tc) {
+    const bool ax = tx <= ty && tx <= tz, ay = !ax && ty <= tz, az = !ax && !ay;
+    w.cx += ax ? (w.r.dx > 0.f ? 1 : -1) : 0;
+    w.cy += ay ? (w.r.dy > 0.f ? 1 : -1) : 0;
+    w.cz += az ? (w.r.dz > 0.f ? 1 : -1) : 0;
+    if (tc > w.r.len || (unsigned)w.cx >= (unsigned)p.dims[0] || (unsigned)w.cy >= (unsigned)p.dims[1] ||
+        (unsigned)w.cz >= (unsigned)p.dims[2])
+        return false;
+    walk_enter(p, w, (w.cz * p.dims[1] + w.cy) * p.dims[0] + w.cx);
+    return true;
+}
+
+template <class GP>
+__device__ __forceinline__ bool walk_step(const GP& p, Walk& w) {
+    float tx, ty, tz;
+    next_crossings(p, w, tx, ty, tz);
+    return walk_cross(p, w, tx, ty, tz, fminf(tx, fminf(ty, tz)));
+}
+
+// walk_step unless the crossing lies at or beyond parameter `stop`: 0 = the segment or the grid ends there, 1 = the
+// next cell was entered, 2 = stopped before a crossing at or beyond `stop`.
+template <class GP>
+__device__ __forceinline__ int walk_step_until(const GP& p, Walk& w, float stop) {
     float tx, ty, tz;
     next_crossings(p, w, tx, ty, tz);
     const float tc = fminf(tx, fminf(ty, tz));
-    if (tc > w.t1) return 0;
+    if (tc > w.r.len) return 0;
     if (tc >= stop) return 2;
-    bool done;
-    if (tx <= ty && tx <= tz) {
-        w.cx += w.r.dx > 0.f ? 1 : -1;
-        done = w.cx < 0 || w.cx >= p.dims[0];
-    } else if (ty <= tz) {
-        w.cy += w.r.dy > 0.f ? 1 : -1;
-        done = w.cy < 0 || w.cy >= p.dims[1];
-    } else {
-        w.cz += w.r.dz > 0.f ? 1 : -1;
-        done = w.cz < 0 || w.cz >= p.dims[2];
-    }
-    if (--w.guard < 0) {  // a monotone walk visits at most dims[0] + dims[1] + dims[2] cells
-        if (err) atomicOr(err, 2u);
-        done = true;
-    }
-    if (done) return 0;
-    walk_enter(p, w, (w.cz * p.dims[1] + w.cy) * p.dims[0] + w.cx);
-    return 1;
-}
-
-// Crosses the nearest cell boundary; false when the segment or the grid ends there.
-template <class GP>
-__device__ __forceinline__ bool walk_step(const GP& p, Walk& w, unsigned int* err) {
-    float tx, ty, tz;
-    next_crossings(p, w, tx, ty, tz);
-    bool done;
-    if (tx <= ty && tx <= tz) {
-        w.cx += w.r.dx > 0.f ? 1 : -1;
-        done = tx > w.t1 || w.cx < 0 || w.cx >= p.dims[0];
-    } else if (ty <= tz) {
-        w.cy += w.r.dy > 0.f ? 1 : -1;
-        done = ty > w.t1 || w.cy < 0 || w.cy >= p.dims[1];
-    } else {
-        w.cz += w.r.dz > 0.f ? 1 : -1;
-        done = tz > w.t1 || w.cz < 0 || w.cz >= p.dims[2];
-    }
-    if (--w.guard < 0) {  // a monotone walk visits at most dims[0] + dims[1] + dims[2] cells
-        if (err) atomicOr(err, 2u);
-        done = true;
-    }
-    if (done) return false;
-    walk_enter(p, w, (w.cz * p.dims[1] + w.cy) * p.dims[0] + w.cx);
-    return true;
+    return walk_cross(p, w, tx, ty, tz, tc) ? 1 : 0;
 }
 
 }  // namespace lyem

@@ -356,7 +356,8 @@ typedef struct lyem_batch_config {
  *   e_p(f) = sum_n S1_f(n, p).
  * lyem_batch_workspace: bytes of the workspace (0: invalid arguments).
  * lyem_batch_items: work items of the launch (per kind: three visibility
- *   stages, scatter fields, sink fields), or minus a status.
+ *   stages, scatter fields, sink fields; a launch may take an item in
+ *   parts), or minus a status.
  * lyem_batch_prepare: writes the scene table, the work list and the
  *   frequency tables into the workspace (256-byte aligned); host -> device
  *   copies, synchronous with the stream.  Repeat after any change of scenes,

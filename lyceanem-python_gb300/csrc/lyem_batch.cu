@@ -20,7 +20,8 @@
 //            elements) on the same sink; each lane stores its sink's visibility of
 //            the chunk as bits of a sink-major mask (one 32-bit word per 32 sources);
 //   W items  e_p(f) for a run of (scatter point, frequency group) slots;
-//   E items  E_f(m) for a run of (sink, frequency group) slots.
+//   E items  E_f(m) for a run of (sink, frequency group) slots; both taken 32
+//            slots at a time, the lanes of a point sharing its pairs' set-up.
 // The queue holds every V item, then every W item, then every E item.  A W
 // item needs its scene's sources -> scatter visibility; an E item needs the
 // two other visibility stages and all W items of its scene.  They wait on the
@@ -244,113 +245,172 @@ __device__ void vis_item(const BatchParams& P, const DevScene& S, const GridView
 
 // ---------------------------------------------------------------- field items
 
-// Adds one visible pair o -> (e, normal nrm) at frequencies f0 .. f0+cnt-1 to acc.
-// Direct form (BOUNCE false): excitation E (6 floats) for every frequency.
-// Bounce form: excitation and weight e_p(f) read from wrow[6 j .. 6 j + 5].
+// What a pair o -> (e, normal nrm) contributes at every frequency.
+struct PairCommon {
+    float v[6];            // direct form: E - (E.d) d of the excitation E; bounce form: direction d
+    int n;                 // bounce form: the source's row
+    float sc, a_re;        // -(1/2pi) (n.d) exp(-alpha r) / r, -alpha - 1/r
+    float rh, rl;          // path length r in float-float
+    float zre, zim;        // exp(-j dbeta r), the rotation of one frequency step
+};
+
 template <int FG, bool BOUNCE>
-__device__ __forceinline__ void pair_freqs(const BatchParams& P, float ox, float oy, float oz, float ex, float ey,
-                                           float ez, float nx, float ny, float nz, const float* E, const float* wrow,
-                                           float2 b0, int f0, int cnt, float (&acc)[6 * FG]) {
+__device__ __forceinline__ PairCommon pair_common(const BatchParams& P, const float* spos, const float* src_E,
+                                                  long long n, float ex, float ey, float ez, float nx, float ny,
+                                                  float nz) {
+    PairCommon c;
+    const float* so = spos + 3 * n;
+    const float ox = __ldg(so), oy = __ldg(so + 1), oz = __ldg(so + 2);
     const Ray r = make_ray(ox, oy, oz, ex, ey, ez);
     const float inv_r = 1.0f / r.len;
     const float mag = expf(-P.alpha * r.len) * inv_r;
-    const float a_re = -P.alpha - inv_r;
+    c.a_re = -P.alpha - inv_r;
     const float nd = nx * r.dx + ny * r.dy + nz * r.dz;
-    const float sc = -0.15915494309189535f * nd * mag;  // -(1/2pi) (n.d) exp(-alpha r)/r
-    float rh, rl;
-    ff_length(ox, oy, oz, ex, ey, ez, rh, rl);
-    // both phases with what their FP32 rounding drops: the rotation below multiplies that of the step up to FG - 1 times
-    float sn, cs, rem;
-    const float ph = ff_phase_parts(b0.x, b0.y, rh, rl, rem);
-    sincos_parts(ph, rem, &sn, &cs);
-    float cre = sc * cs, cim = -sc * sn;  // sc exp(-j beta_f0 r)
-    float zre = 1.f, zim = 0.f;
+    c.sc = -0.15915494309189535f * nd * mag;
+    ff_length(ox, oy, oz, ex, ey, ez, c.rh, c.rl);
+    c.zre = 1.f;
+    c.zim = 0.f;
     if (FG > 1) {
-        float zs, zc;
-        const float dph = ff_phase_parts(P.dbeta_ff.x, P.dbeta_ff.y, rh, rl, rem);
+        // with what the FP32 rounding of the phase drops: the rotation multiplies that of the step up to FG - 1 times
+        float zs, zc, rem;
+        const float dph = ff_phase_parts(P.dbeta_ff.x, P.dbeta_ff.y, c.rh, c.rl, rem);
         sincos_parts(dph, rem, &zs, &zc);
-        zre = zc;
-        zim = -zs;
+        c.zre = zc;
+        c.zim = -zs;
     }
-    float el[6];
-    if (!BOUNCE) {  // E_L = E - (E.d) d, the same for every frequency
-        const float ed_re = E[0] * r.dx + E[2] * r.dy + E[4] * r.dz;
-        const float ed_im = E[1] * r.dx + E[3] * r.dy + E[5] * r.dz;
-        el[0] = E[0] - ed_re * r.dx; el[1] = E[1] - ed_im * r.dx;
-        el[2] = E[2] - ed_re * r.dy; el[3] = E[3] - ed_im * r.dy;
-        el[4] = E[4] - ed_re * r.dz; el[5] = E[5] - ed_im * r.dz;
+    c.n = (int)n;
+    if (BOUNCE) {
+        c.v[0] = r.dx; c.v[1] = r.dy; c.v[2] = r.dz;
+        c.v[3] = c.v[4] = c.v[5] = 0.f;
+    } else {
+        const float2* e2 = reinterpret_cast<const float2*>(src_E + 6 * n);
+        const float2 e0 = __ldg(e2), e1 = __ldg(e2 + 1), e3 = __ldg(e2 + 2);
+        const float ed_re = e0.x * r.dx + e1.x * r.dy + e3.x * r.dz;
+        const float ed_im = e0.y * r.dx + e1.y * r.dy + e3.y * r.dz;
+        c.v[0] = e0.x - ed_re * r.dx; c.v[1] = e0.y - ed_im * r.dx;
+        c.v[2] = e1.x - ed_re * r.dy; c.v[3] = e1.y - ed_im * r.dy;
+        c.v[4] = e3.x - ed_re * r.dz; c.v[5] = e3.y - ed_im * r.dz;
     }
+    return c;
+}
+
+// The values a lane set up, through shared memory: three float4 a lane.
+template <bool BOUNCE>
+__device__ __forceinline__ void put_pair(float4 (*ent)[32], int lane, const PairCommon& c) {
+    ent[0][lane] = make_float4(c.v[0], c.v[1], c.v[2], c.sc);
+    ent[1][lane] = make_float4(BOUNCE ? __int_as_float(c.n) : c.v[3], c.v[4], c.v[5], c.a_re);
+    ent[2][lane] = make_float4(c.rh, c.rl, c.zre, c.zim);
+}
+
+template <bool BOUNCE>
+__device__ __forceinline__ PairCommon get_pair(const float4 (*ent)[32], int lane) {
+    const float4 a = ent[0][lane], b = ent[1][lane], d = ent[2][lane];
+    PairCommon c;
+    c.v[0] = a.x; c.v[1] = a.y; c.v[2] = a.z; c.v[3] = b.x; c.v[4] = b.y; c.v[5] = b.z;
+    c.n = BOUNCE ? __float_as_int(b.x) : 0;
+    c.sc = a.w; c.a_re = b.w;
+    c.rh = d.x; c.rl = d.y; c.zre = d.z; c.zim = d.w;
+    return c;
+}
+
+// Adds the pair at frequencies f0 .. f0+cnt-1 to acc.
+// Bounce form: excitation and weight e_p(f) read from row n of w.
+template <int FG, bool BOUNCE>
+__device__ __forceinline__ void pair_freqs(const BatchParams& P, const PairCommon& c, const float* w, float2 b0, int f0,
+                                           int cnt, float (&acc)[6 * FG]) {
+    float sn, cs, rem;
+    const float ph = ff_phase_parts(b0.x, b0.y, c.rh, c.rl, rem);
+    sincos_parts(ph, rem, &sn, &cs);
+    float cre = c.sc * cs, cim = -c.sc * sn;  // sc exp(-j beta_f0 r)
+    const float* wrow = BOUNCE ? w + ((long long)c.n * P.n_freq + f0) * 6 : nullptr;
 #pragma unroll
     for (int j = 0; j < FG; ++j) {
         if (j < cnt) {
             const float b = __ldg(P.beta_f + f0 + j);
             // loss = (a_re - j beta) * c
-            const float lre = a_re * cre + b * cim;
-            const float lim = a_re * cim - b * cre;
+            const float lre = c.a_re * cre + b * cim;
+            const float lim = c.a_re * cim - b * cre;
             if (!BOUNCE) {
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    acc[6 * j + 2 * k] += el[2 * k] * lre - el[2 * k + 1] * lim;
-                    acc[6 * j + 2 * k + 1] += el[2 * k] * lim + el[2 * k + 1] * lre;
+                    acc[6 * j + 2 * k] += c.v[2 * k] * lre - c.v[2 * k + 1] * lim;
+                    acc[6 * j + 2 * k + 1] += c.v[2 * k] * lim + c.v[2 * k + 1] * lre;
                 }
             } else {
                 const float2 w0 = *reinterpret_cast<const float2*>(wrow + 6 * j);
                 const float2 w1 = *reinterpret_cast<const float2*>(wrow + 6 * j + 2);
                 const float2 w2 = *reinterpret_cast<const float2*>(wrow + 6 * j + 4);
                 const float e[6] = {w0.x, w0.y, w1.x, w1.y, w2.x, w2.y};
-                const float ed_re = e[0] * r.dx + e[2] * r.dy + e[4] * r.dz;
-                const float ed_im = e[1] * r.dx + e[3] * r.dy + e[5] * r.dz;
-                const float dd[3] = {r.dx, r.dy, r.dz};
+                const float ed_re = e[0] * c.v[0] + e[2] * c.v[1] + e[4] * c.v[2];
+                const float ed_im = e[1] * c.v[0] + e[3] * c.v[1] + e[5] * c.v[2];
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    const float pr = e[2 * k] - ed_re * dd[k], pi = e[2 * k + 1] - ed_im * dd[k];
+                    const float pr = e[2 * k] - ed_re * c.v[k], pi = e[2 * k + 1] - ed_im * c.v[k];
                     const float tr = pr * lre - pi * lim, ti = pr * lim + pi * lre;  // S2 component
                     acc[6 * j + 2 * k] += e[2 * k] * tr - e[2 * k + 1] * ti;      // weighted by e_p
                     acc[6 * j + 2 * k + 1] += e[2 * k] * ti + e[2 * k + 1] * tr;
                 }
             }
-            const float nre = cre * zre - cim * zim;
-            cim = cre * zim + cim * zre;
+            const float nre = cre * c.zre - cim * c.zim;
+            cim = cre * c.zim + cim * c.zre;
             cre = nre;
         }
     }
 }
 
+// How the lanes of a warp set up the pairs of its sinks (field_item).  A pair's direction, distance, amplitude and
+// transverse excitation are the same at every frequency, and cost about as much as three frequencies: with more than
+// kAloneGroups frequency groups a sink, `per` pairs of each of the warp's sinks are set up at a time, a pair a lane, and
+// every lane of the sink then adds them at its own frequencies.  This lane sets up number `rank` of a sink whose bits
+// lane `at` holds, and reads those of its own sink from the lanes `from` .. `from` + per - 1.  With fewer groups each
+// lane sets up its own pairs (per = 1): no lane waits for another then.
+// 8 scenes, 1e8 pairs, one frequency a lane, 2 / 3 / 4 / 8 / 16 / 64 frequencies, each alone 27.5 / 28.9 / 31.4 / 33.3
+// / 56 / 134 ms, shared 36.4 / 36.7 / 31.6 / 28.9 / 29.8 / 35.5 ms.
+constexpr int kAloneGroups = 4;
+struct Share {
+    int per, rank, at, from;
+    bool sets;
+};
+
 // Sums the pairs of one stage into the thread's accumulator in shared memory
 // (sacc[k * kBT + tid], k < 6 FG): per 32 sources in registers, then added.
+// Called by all lanes of a warp; ok: the lane has a sink.  (x, y, z) and normal:
+// the sink whose pairs the lane sets up.
 template <int FG, bool BOUNCE>
 __device__ __forceinline__ void field_stage(const BatchParams& P, const unsigned int* row, long long words,
                                             const float* spos, const float* src_E, const float* w, bool ok, float ex,
                                             float ey, float ez, float nx, float ny, float nz, float2 b0, int f0,
-                                            int cnt, float* sacc) {
+                                            int cnt, const Share& sh, float4 (*ent)[32], float* sacc) {
+    const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x;
-    if (!ok) return;
     for (long long wi = 0; wi < words; ++wi) {
-        unsigned int bits = row[wi];
-        if (!bits) continue;
+        unsigned int bits = ok ? row[wi] : 0u;
+        if (!__any_sync(full, bits != 0)) continue;
         float acc[6 * FG];
 #pragma unroll
         for (int k = 0; k < 6 * FG; ++k) acc[k] = 0.f;
-        while (bits) {
-            const int j = __ffs(bits) - 1;
-            bits &= bits - 1;
-            const long long n = (wi << 5) + j;
-            const float* so = spos + 3 * n;
-            const float ox = __ldg(so), oy = __ldg(so + 1), oz = __ldg(so + 2);
-            if (!BOUNCE) {
-                float E[6];
-                const float2* e2 = reinterpret_cast<const float2*>(src_E + 6 * n);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float2 v = __ldg(e2 + k);
-                    E[2 * k] = v.x;
-                    E[2 * k + 1] = v.y;
-                }
-                pair_freqs<FG, false>(P, ox, oy, oz, ex, ey, ez, nx, ny, nz, E, nullptr, b0, f0, cnt, acc);
-            } else {
-                const float* wrow = w + (n * P.n_freq + f0) * 6;
-                pair_freqs<FG, true>(P, ox, oy, oz, ex, ey, ez, nx, ny, nz, nullptr, wrow, b0, f0, cnt, acc);
+        if (sh.per == 1) {
+            while (bits) {
+                const int j = __ffs(bits) - 1;
+                bits &= bits - 1;
+                const PairCommon c = pair_common<FG, BOUNCE>(P, spos, src_E, (wi << 5) + j, ex, ey, ez, nx, ny, nz);
+                pair_freqs<FG, BOUNCE>(P, c, w, b0, f0, cnt, acc);
             }
+        } else {
+            do {
+                unsigned int mine = __shfl_sync(full, bits, sh.at);  // without its `rank` lowest bits
+                for (int k = 0; k < sh.rank; ++k) mine &= mine - 1;
+                const int j = mine ? __ffs(mine) - 1 : 0;
+                if (sh.sets && mine)
+                    put_pair<BOUNCE>(ent, tid & 31, pair_common<FG, BOUNCE>(P, spos, src_E, (wi << 5) + j, ex, ey, ez, nx, ny, nz));
+                const int take = min(__popc(bits), sh.per);
+                __syncwarp();
+                for (int i = 0; i < take; ++i)
+                    pair_freqs<FG, BOUNCE>(P, get_pair<BOUNCE>(ent, sh.from + i), w, b0, f0, cnt, acc);
+                __syncwarp();
+                const int last = __shfl_sync(full, j, sh.from + max(take - 1, 0));
+                if (take) bits &= ~((2u << last) - 1u);
+            } while (__any_sync(full, bits != 0));
         }
 #pragma unroll
         for (int k = 0; k < 6 * FG; ++k) sacc[k * kBT + tid] += acc[k];
@@ -360,8 +420,8 @@ __device__ __forceinline__ void field_stage(const BatchParams& P, const unsigned
 // One warp's 32 consecutive slots (chunk of the scene's slot list).
 template <int FG>
 __device__ void field_item(const BatchParams& P, const DevScene& S, int scene, int kind, long long chunk,
-                           float* sacc) {
-    const int tid = threadIdx.x;
+                           float4 (*ent)[32], float* sacc) {
+    const int tid = threadIdx.x, lane = tid & 31;
     const int G = P.n_groups;
     const bool at_sinks = kind == kFieldE;
     const long long nk = at_sinks ? P.n_snk : S.n_scat;
@@ -371,21 +431,32 @@ __device__ void field_item(const BatchParams& P, const DevScene& S, int scene, i
     const int f0 = g * FG;
     const int cnt = min(FG, P.n_freq - f0);
     const bool ok = ms < nk && cnt > 0;
+    const int m0 = __shfl_sync(0xffffffffu, (int)ms, 0), g0 = __shfl_sync(0xffffffffu, g, 0);
+    const int sinks = (g0 + 31) / G + 1;
+    Share sh;
+    sh.per = 32 / sinks;
+    const int own = lane / sh.per;
+    sh.rank = lane - own * sh.per;
+    sh.sets = own < sinks && m0 + own < nk;
+    sh.at = sh.sets ? max(own * G - g0, 0) : lane;
+    sh.from = ((int)ms - m0) * sh.per;
+    if (G <= kAloneGroups) sh.per = 1;  // (the warp may hold up to 32 sinks)
+    const long long ks = sh.per == 1 ? ms : (long long)m0 + own;
 #pragma unroll
     for (int k = 0; k < 6 * FG; ++k) sacc[k * kBT + tid] = 0.f;
     float ex = 0.f, ey = 0.f, ez = 0.f, nx = 0.f, ny = 0.f, nz = 0.f;
     float2 b0 = make_float2(0.f, 0.f);
-    if (ok) {
-        const float* kp = (at_sinks ? P.snk_pos : S.scat_pos) + 3 * ms;
-        const float* kn = (at_sinks ? P.snk_nrm : S.scat_nrm) + 3 * ms;
+    if (ok) b0 = __ldg(P.beta_ff + f0);
+    if (sh.per == 1 ? ok : sh.sets) {
+        const float* kp = (at_sinks ? P.snk_pos : S.scat_pos) + 3 * ks;
+        const float* kn = (at_sinks ? P.snk_nrm : S.scat_nrm) + 3 * ks;
         ex = __ldg(kp); ey = __ldg(kp + 1); ez = __ldg(kp + 2);
         nx = __ldg(kn); ny = __ldg(kn + 1); nz = __ldg(kn + 2);
-        b0 = __ldg(P.beta_ff + f0);
     }
     if (!at_sinks) {
         const long long words = S.mask_words[kVisScat];
         field_stage<FG, false>(P, S.mask[kVisScat] + ms * words, words, S.src_pos, S.src_E, nullptr, ok, ex, ey, ez,
-                               nx, ny, nz, b0, f0, cnt, sacc);
+                               nx, ny, nz, b0, f0, cnt, sh, ent, sacc);
         if (ok) {
             float* out = S.w + (ms * P.n_freq + f0) * 6;
             for (int k = 0; k < 6 * cnt; ++k) out[k] = sacc[k * kBT + tid];
@@ -395,12 +466,12 @@ __device__ void field_item(const BatchParams& P, const DevScene& S, int scene, i
     {
         const long long words = S.mask_words[kVisDirect];
         field_stage<FG, false>(P, S.mask[kVisDirect] + ms * words, words, S.src_pos, S.src_E, nullptr, ok, ex, ey,
-                               ez, nx, ny, nz, b0, f0, cnt, sacc);
+                               ez, nx, ny, nz, b0, f0, cnt, sh, ent, sacc);
     }
     if (S.n_scat > 0) {
         const long long words = S.mask_words[kVisBounce];
         field_stage<FG, true>(P, S.mask[kVisBounce] + ms * words, words, S.scat_pos, nullptr, S.w, ok, ex, ey, ez,
-                              nx, ny, nz, b0, f0, cnt, sacc);
+                              nx, ny, nz, b0, f0, cnt, sh, ent, sacc);
     }
     if (ok) {
         const long long m = P.snk_id ? (long long)__ldg(P.snk_id + ms) : ms;
@@ -425,6 +496,7 @@ template <bool CULL, int FG, int MINB>
 __global__ void __launch_bounds__(kBT, MINB) batch_kernel(const BatchParams P) {
     extern __shared__ float sacc[];
     __shared__ GridView s_grid[kBT / 32];
+    __shared__ float4 s_ent[kBT / 32][3][32];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     unsigned nxt = 0;
@@ -469,7 +541,7 @@ __global__ void __launch_bounds__(kBT, MINB) batch_kernel(const BatchParams P) {
                                part * (kWarpSinks / P.split), (part + 1) * (kWarpSinks / P.split));
             else
                 for (int t = 0; t < b; ++t)  // b consecutive 32-slot chunks
-                    field_item<FG>(P, S, scene, kind, (long long)a + t, sacc);
+                    field_item<FG>(P, S, scene, kind, (long long)a + t, s_ent[wid], sacc);
         }
         __threadfence();
         __syncwarp();
@@ -485,6 +557,7 @@ struct Plan {
     std::vector<int4> items;
     std::vector<size_t> off_mask[3], off_w;
     std::vector<int> expect;  // [n_scenes][kKinds]
+    long long count[kKinds] = {};  // items of each kind (items holds the field items' parts)
     size_t off_ctrl = 0, ctrl_bytes = 0, off_scenes = 0, off_items = 0, off_beta = 0, off_betaf = 0, total = 0;
 };
 
@@ -559,6 +632,7 @@ int make_plan(const lyem_batch_scene* sc, int n_scenes, long long n_snk, int n_f
             for (long long t = 0; t < nk; t += kWarpSinks) pl.items.push_back(make_int4(stage, s, (int)n0, (int)t));
         pl.expect[(size_t)s * kKinds + stage] =
             (int)(((ns + chunk - 1) / chunk) * ((nk + kWarpSinks - 1) / kWarpSinks));
+        pl.count[stage] += pl.expect[(size_t)s * kKinds + stage];
     };
     for (int s : order) {
         const long long N = sc[s].n_src, P = sc[s].n_scat;
@@ -567,18 +641,22 @@ int make_plan(const lyem_batch_scene* sc, int n_scenes, long long n_snk, int n_f
         add_vis(s, kVisBounce, P, n_snk);
     }
     // A field item is a run of 32-slot chunks (slot = point * groups + group),
-    // long enough for about kItemPairs candidate (pair, group) evaluations, so
-    // that scenes with few sources do not become very many tiny items.
+    // long enough for about kItemPairs candidate (pair, group) evaluations.
+    // The list holds its parts: a chunk each (more where a point has fewer
+    // than 64 sources), since a warp adds a chunk's pairs one behind the other
+    // whatever the number of groups, and long runs left most warps without
+    // work.  8 scenes of up to 178 elements, 1,649 sinks, 8 / 64 frequencies:
+    // whole items 9.0 / 25.8 ms, parts 3.4 / 4.4 ms; 8 of up to 4,096, 4,000
+    // sinks, 16 / 64 frequencies: 35.6 / 72.8 and 29.8 / 35.3 ms.
     auto add_field = [&](int s, int kind, long long nk, long long pairs_per_sink) {
         const long long chunks = (nk * groups + 31) / 32;
         const long long per_chunk = std::max(1LL, pairs_per_sink * 32 / groups);
         const long long k = std::min(64LL, std::max(1LL, (kItemPairs + per_chunk - 1) / per_chunk));
-        int count = 0;
-        for (long long c = 0; c < chunks; c += k) {
-            pl.items.push_back(make_int4(kind, s, (int)c, (int)std::min(k, chunks - c)));
-            ++count;
-        }
-        pl.expect[(size_t)s * kKinds + kind] = count;
+        pl.count[kind] += (chunks + k - 1) / k;
+        const long long part = std::max(1LL, 64 / std::max(1LL, pairs_per_sink));
+        for (long long c = 0; c < chunks; c += part)
+            pl.items.push_back(make_int4(kind, s, (int)c, (int)std::min(part, chunks - c)));
+        pl.expect[(size_t)s * kKinds + kind] = (int)((chunks + part - 1) / part);
     };
     for (int s : order) add_field(s, kFieldW, sc[s].n_scat, sc[s].n_src);
     for (int s : order) add_field(s, kFieldE, n_snk, sc[s].n_src + sc[s].n_scat);
@@ -683,11 +761,12 @@ LYEM_API int64_t lyem_batch_items(const lyem_batch_scene* scenes, int32_t n_scen
     Plan pl;
     const int st = make_plan(scenes, n_scenes, n_snk, n_freq, config, pl);
     if (st != LYEM_OK) return -(int64_t)st;
-    if (per_kind5) {
-        for (int k = 0; k < kKinds; ++k) per_kind5[k] = 0;
-        for (const int4& it : pl.items) per_kind5[it.x] += 1;
+    int64_t total = 0;
+    for (int k = 0; k < kKinds; ++k) {
+        if (per_kind5) per_kind5[k] = pl.count[k];
+        total += pl.count[k];
     }
-    return (int64_t)pl.items.size();
+    return total;
 }
 
 LYEM_API int lyem_batch_prepare(const lyem_batch_scene* scenes, int32_t n_scenes, int64_t n_snk,

@@ -35,21 +35,17 @@ C0 = 299792458.0
 # (frequencies per thread, sources per visibility item, blocks per SM).  Blocks per
 # SM 3, 4, 6 or 8 select kernel variants whose registers are capped for that
 # occupancy; 0 runs the uncapped variant with as many blocks as fit.
-CANDIDATES = [(2, 64, 8), (2, 64, 6), (2, 32, 6), (1, 32, 8), (2, 32, 8), (4, 64, 4), (4, 32, 4), (4, 32, 3), (8, 32, 3)]
+CANDIDATES = [(1, 32, 8), (1, 32, 4), (1, 64, 8), (1, 64, 4), (2, 32, 6), (2, 32, 4), (4, 32, 4)]
 
 
-def default_config(n_freq, pairs, uniform):
-    """Configuration of a batch that is not tuned.  Few frequencies: one per thread (the pair set-up is not shared, so
-    threads go to sinks), and the most warps for the walks.  More: four per thread, which share the set-up, unless the
-    walks dominate (200 million ray pairs and more), which want the warps.  Milliseconds at (2, 64, 8) / (1, 32, 8) /
-    (2, 32, 6) / (4, 32, 4): 8 scenes, 1e8 pairs, 1 frequency 36.9 / 29.4 / 32.3 / 34.3, 4 frequencies 41.5 / 31.7 /
-    34.3 / 38.0, 16 frequencies 59.3 / 56.4 / 47.5 / 45.9, 64 frequencies 131 / 159 / 112 / 81; 24 scenes, 6e8 pairs, 16
-    frequencies 190 / 196 / 183 / 196; 3 small scenes, 7 frequencies 8.5 / 8.3 / 6.7 / 4.4."""
-    if n_freq <= 4 or not uniform:
-        return (1, 32, 8)
-    if n_freq < 32 and pairs >= 2e8:
-        return (2, 32, 6)
-    return (4, 32, 4)
+def default_config(n_freq):
+    """Configuration of a batch that is not tuned: one frequency per thread (the threads of a sink share the set-up of its
+    pairs), with the most warps for the walks up to four frequencies and the most registers for the fields from there on.
+    Milliseconds at (1, 32, 8) / (1, 32, 4) / (2, 32, 6) / (4, 32, 4): 8 scenes, 1e8 pairs, 1 frequency 26.4 / 27.5 / 28.3
+    / 30.3, 4 frequencies 31.4 / 30.2 / 31.0 / 34.1, 16 frequencies 33.8 / 29.9 / 33.4 / 39.8, 64 frequencies 43.9 / 35.3
+    / 38.9 / 46.8; 8 scenes, 8e6 pairs, 1 frequency 2.8 / 2.9 / 3.4 / 3.3, 4 frequencies 2.9 / 3.1 / 3.7 / 3.9, 16
+    frequencies 3.9 / 3.8 / 4.6 / 4.3, 64 frequencies 5.4 / 4.4 / 5.6 / 6.3."""
+    return (1, 32, 8) if n_freq <= 4 else (1, 32, 4)
 
 
 def stratified_subset(scenes, n_sinks, every=4):
@@ -206,7 +202,7 @@ class BatchedScattering:
     # ------------------------------------------------------------ configuration
 
     def _default(self):
-        return default_config(self.n_freq, self.pairs(), self.uniform)
+        return default_config(self.n_freq)
 
     def _cfg(self, c):
         cfg = BatchConfig()

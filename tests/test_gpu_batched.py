@@ -237,3 +237,26 @@ def test_split_visibility_items(copies, n_snk):
         assert rel_err(field[s, 0], out.cpu().numpy()) < 2e-6  # FP32 sums of up to 150 terms in two orders
     st, flags = P.device_errors()
     assert st == 0 and flags == 0
+
+
+@pytest.mark.parametrize("fg,n_freq", [(1, 1), (1, 4), (1, 5), (1, 17), (1, 31), (1, 32), (1, 33), (1, 65), (2, 8), (2, 9),
+                                       (2, 61), (4, 24), (8, 41)])
+def test_shared_pair_setup(fg, n_freq):
+    """Frequency groups on both sides of the line from which the lanes of a sink share its pairs' set-up, and that split
+    a warp between sinks unevenly: first, middle and last frequency against the per-scene pair stages."""
+    B, P, SC = _mods()
+    scenes, snk, snk_n = _small_batch(n_snk=83)
+    freqs = np.linspace(25e9, 29e9, n_freq) if n_freq > 1 else np.array([27e9])
+    b = B.BatchedScattering(scenes, snk, snk_n, freqs, cell_scale=1.5, config=(fg, 32, 4))
+    field = b.run().cpu().numpy()
+    betas = B.betas_of(freqs)
+    for s, sc in enumerate(scenes):
+        tris = P.pack_triangles(sc.verts, sc.faces)
+        for f in sorted({0, n_freq // 2, n_freq - 1}):
+            kw = dict(beta=float(betas[f]), tris=tris)
+            out = P.pair_stage(sc.src, sc.E, snk, snk_n, **kw).sink
+            if len(sc.scat):
+                e_p = P.pair_stage(sc.src, sc.E, sc.scat, sc.scat_n, **kw).sink
+                P.pair_stage(sc.scat, e_p, snk, snk_n, src_W=e_p, sink_out=out, accumulate=True, **kw)
+            assert rel_err(field[s, f], out.cpu().numpy()) < 2e-6  # FP32 sums of up to 150 terms in two orders
+    assert P.device_errors() == (0, 0)

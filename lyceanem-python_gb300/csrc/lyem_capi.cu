@@ -124,13 +124,18 @@ void lyem::record_cuda_error(cudaError_t e) { g_last_cuda_error = (int)e; }
 // Sources per thread block when the caller passes 0.  Brute force: as many
 // as keep about four waves of blocks in flight (the triangle tiles are
 // re-staged per block).  Grid: 16, or 64 for 16,384 sources and more, fewer
-// when that would leave under four waves.  On the 28 GHz one-bounce scene the
-// scatter->sink stage (50,000 sources) measured 539.7 / 536.8 / 537.7 ms at
-// 16 / 32 / 64, and 64 writes a quarter of the per-chunk partial sums of 16;
-// the 1,024-source stages were faster at 16.
+// when that would leave under eight waves of sixteen blocks an SM: the blocks
+// of a stage end at very different times (sinks over open ground, sinks behind
+// the clutter), and with one or two waves its last blocks run alone.  Lockstep,
+// with two waves -> with eight: 500 sources to 4,186 sinks 0.345 -> 0.326 ms,
+// 2,000 to 2,701 2.01 -> 1.51 (40,000 triangles), 2,000 to 4,186 1.13 -> 1.02,
+// 1,000 to 7,381 1.28 -> 1.05, 5,000 to 7,381 7.6 -> 7.2; 16 waves gain no more.
+// On the 28 GHz one-bounce scene the scatter->sink stage (50,000 sources)
+// measured 539.7 / 536.8 / 537.7 ms at 16 / 32 / 64, and 64 writes a quarter of
+// the per-chunk partial sums of 16; the 1,024-source stages were faster at 16.
 int lyem::auto_src_chunk(long long n_src, long long n_snk, bool grid) {
     const long long tiles = (n_snk + stage_block_threads() - 1) / stage_block_threads();
-    const long long waves = (long long)device_sm_count() * 8 * 4;
+    const long long waves = (long long)device_sm_count() * (grid ? 16 * 8 : 8 * 4);
     long long c;
     if (grid) {
         c = n_src >= 16384 ? 64 : 16;

@@ -21,7 +21,9 @@
 //            the chunk as bits of a sink-major mask (one 32-bit word per 32 sources);
 //   W items  e_p(f) for a run of (scatter point, frequency group) slots;
 //   E items  E_f(m) for a run of (sink, frequency group) slots; both taken 32
-//            slots at a time, the lanes of a point sharing its pairs' set-up.
+//            slots at a time, the lanes of a point sharing its pairs' set-up,
+//            or, with few groups, a point at a time, its lanes sharing its
+//            sources.
 // The queue holds every V item, then every W item, then every E item.  A W
 // item needs its scene's sources -> scatter visibility; an E item needs the
 // two other visibility stages and all W items of its scene.  They wait on the
@@ -116,9 +118,16 @@ struct BatchParams {
 
 // ---------------------------------------------------------------- queue
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+// Completion counters.  The walks live on what the SM's L1 holds of the grid, and an acquire (a load of that kind, or
+// __threadfence) drops all of it: items end with a release, and a wait polls with relaxed loads, sparingly, and fences
+// once at its end.
+__device__ __forceinline__ void add_release(unsigned* p, unsigned v) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
     unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -126,10 +135,12 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 __device__ bool wait_count(const unsigned* ctr, unsigned target) {
     if (target == 0) return true;
     const long long t0 = clock64();
+    unsigned pause = 500;
     while (true) {
-        if (ld_acquire(ctr) >= target) return true;
+        if (ld_relaxed(ctr) >= target) return true;
         if (clock64() - t0 > kWaitCycles) return false;
-        __nanosleep(200);
+        __nanosleep(pause);
+        pause = min(pause * 2u, 4000u);
     }
 }
 
@@ -137,10 +148,15 @@ __device__ bool wait_deps(const BatchParams& P, int kind, int scene) {
     const DevScene& S = P.scenes[scene];
     const unsigned* d = P.done + (long long)scene * kKinds;
     const unsigned parts = (unsigned)P.split;
-    if (kind == kFieldW) return wait_count(d + kVisScat, (unsigned)S.expect[kVisScat] * parts);
-    bool ok = wait_count(d + kVisDirect, (unsigned)S.expect[kVisDirect] * parts);
-    ok = ok && wait_count(d + kVisBounce, (unsigned)S.expect[kVisBounce] * parts);
-    ok = ok && wait_count(d + kFieldW, (unsigned)S.expect[kFieldW]);
+    bool ok;
+    if (kind == kFieldW) {
+        ok = wait_count(d + kVisScat, (unsigned)S.expect[kVisScat] * parts);
+    } else {
+        ok = wait_count(d + kVisDirect, (unsigned)S.expect[kVisDirect] * parts);
+        ok = ok && wait_count(d + kVisBounce, (unsigned)S.expect[kVisBounce] * parts);
+        ok = ok && wait_count(d + kFieldW, (unsigned)S.expect[kFieldW]);
+    }
+    __threadfence();
     return ok;
 }
 
@@ -152,63 +168,42 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 
 // ---------------------------------------------------------------- V items
 
-// The scene's grid parameters are read from shared memory (sgrid, filled by
-// the caller) rather than held in registers through the walk.
-template <bool CULL>
-__device__ void vis_item(const BatchParams& P, const DevScene& S, const GridView& G, int scene, int stage,
-                         long long n0, long long m0, int i0, int i1) {
+// The scene's grid parameters are read from shared memory (filled by the
+// caller) rather than held in registers through the walk.
+// TURNED: the lanes are 32 of the chunk's sources and the warp walks to one sink of i0 .. i1 - 1 after the other;
+// otherwise they are the 32 sinks and it walks from one source after the other.
+template <bool CULL, bool TURNED>
+__device__ __forceinline__ void vis_walks(const BatchParams& P, const GridView& G, const float* spos, const int* sid, long long n0,
+                          int nsrc, const float* kpos, const int* kid, long long m0, long long nk, int i0, int i1,
+                          unsigned int* mask, long long words, unsigned int& vis, unsigned int& tests) {
     const int lane = threadIdx.x & 31;
-    const float* spos = stage == kVisBounce ? S.scat_pos : S.src_pos;
-    const long long ns = stage == kVisBounce ? S.n_scat : S.n_src;
-    const int* sid = stage == kVisBounce ? S.scat_id : nullptr;
-    const float* kpos = stage == kVisScat ? S.scat_pos : P.snk_pos;
-    const long long nk = stage == kVisScat ? S.n_scat : P.n_snk;
-    const int* kid = stage == kVisScat ? S.scat_id : P.snk_id;
-    const long long ms = m0 + lane;
-    const bool ok = ms < nk;
-    const long long rem = ns - n0;
-    const int nsrc = (int)(rem < P.src_chunk ? rem : P.src_chunk);
-    long long m_id = -1;
-    float ex = 0.f, ey = 0.f, ez = 0.f;
-    if (ok) {
-        m_id = kid ? (long long)__ldg(kid + ms) : ms;
-        ex = __ldg(kpos + 3 * ms);
-        ey = __ldg(kpos + 3 * ms + 1);
-        ez = __ldg(kpos + 3 * ms + 2);
-    }
-    unsigned long long vis = 0;
-    unsigned int tests = 0;  // diagnostic count of one lane (64 rays at most); wraps only past 2^32 tests
+    const bool ok = m0 + lane < nk;
+    const int last = TURNED ? (int)min((long long)i1, nk - m0) : 0;
     Walk w;
-    // The element stages turn the warp round: the lanes are 32 of the chunk's sources (an array's elements) and the
-    // warp walks to one sink after the other, so its rays cross the same cells (as grid_transposed_kernel does; 8 scenes
-    // of up to 3,969 elements, 16 frequencies: 64.0 -> 59.3 ms at (2, 64, 8), 57.1 -> 46.6 at (2, 32, 6)).
-    // Scatter points as sources are turned for few sinks, which lie too far apart to share a walk (the rule of
-    // propagation.scatter_schedule), and where items are split; a part of an item holds its sinks i0 .. i1 - 1.
-    const bool turned = stage != kVisBounce || P.turn_all;
     for (int g = 0; g < nsrc; g += 32) {
-        const int first = turned ? i0 : 0, last = turned ? i1 : min(32, nsrc - g);
-        const bool n_ok = g + lane < nsrc;
-        unsigned int word = 0;
-        float lx = ex, ly = ey, lz = ez;  // the lane's end point: its sink, or its source where turned
-        if (turned) {
-            const float* so = spos + 3 * (n0 + g + (n_ok ? lane : 0));
-            lx = __ldg(so); ly = __ldg(so + 1); lz = __ldg(so + 2);
+        const long long mine = TURNED ? n0 + g + lane : m0 + lane;  // the lane's point
+        const bool has = TURNED ? g + lane < nsrc : ok;
+        float lx = 0.f, ly = 0.f, lz = 0.f;
+        int id = -1;
+        if (has) {
+            const float* l = (TURNED ? spos : kpos) + 3 * mine;
+            lx = __ldg(l); ly = __ldg(l + 1); lz = __ldg(l + 2);
+            const int* ids = TURNED ? sid : kid;
+            id = ids ? __ldg(ids + mine) : (int)mine;
         }
-        for (int i = first; i < last; ++i) {
-            const long long n = n0 + g + (turned ? (n_ok ? lane : 0) : i);
-            const long long k = turned ? m0 + i : ms;
-            if (turned && k >= nk) break;  // the same in every lane
-            const bool mine = turned ? n_ok : ok;
-            bool seen = mine;
-            const long long n_id = sid ? (long long)__ldg(sid + n) : n;
-            const long long k_id = !turned ? m_id : kid ? (long long)__ldg(kid + k) : k;
-            if (mine && !(P.skip_diag && n_id == k_id)) {  // (a skipped pair is not tested: visible)
-                const float* o = turned ? kpos + 3 * k : spos + 3 * n;
+        if (!P.skip_diag) id = -1;
+        unsigned int word = 0;
+        for (int i = TURNED ? i0 : 0; i < (TURNED ? last : min(32, nsrc - g)); ++i) {
+            const long long u = TURNED ? m0 + i : n0 + g + i;  // the point all lanes walk to or from
+            const int* ids = TURNED ? kid : sid;
+            bool hit = !has;
+            if (has && id != (ids ? __ldg(ids + u) : (int)u)) {  // (a skipped pair is not tested: visible)
+                const float* o = (TURNED ? kpos : spos) + 3 * u;
                 const float ux = __ldg(o), uy = __ldg(o + 1), uz = __ldg(o + 2);
-                if (walk_begin<CULL>(G, w, turned ? lx : ux, turned ? ly : uy, turned ? lz : uz, turned ? ux : lx,
-                                     turned ? uy : ly, turned ? uz : lz)) {
-                    bool hit = false;
-                    while (true) {
+                if (TURNED) walk_ray<CULL>(w, lx, ly, lz, ux, uy, uz);
+                else walk_ray<CULL>(w, ux, uy, uz, lx, ly, lz);
+                if (walk_setup(G, w)) {
+                    while (!hit) {
                         while (w.q < w.q1) {
                             ++tests;
                             if (walk_test<CULL>(G, w)) {
@@ -218,25 +213,47 @@ __device__ void vis_item(const BatchParams& P, const DevScene& S, const GridView
                         }
                         if (hit || !walk_step(G, w)) break;
                     }
-                    seen = !hit;
                 }
             }
-            if (turned) {
-                const unsigned int b = __ballot_sync(0xffffffffu, seen);
+            if (TURNED) {
+                const unsigned int b = __ballot_sync(0xffffffffu, !hit);
                 if (lane == i) word = b;
-            } else if (seen) {
-                word |= 1u << i;
+            } else {
+                __syncwarp();
+                if (!hit) word |= 1u << i;
             }
         }
-        if (ok && (!turned || (lane >= i0 && lane < i1))) {
-            S.mask[stage][ms * S.mask_words[stage] + ((n0 + g) >> 5)] = word;
+        if (ok && (!TURNED || (lane >= i0 && lane < i1))) {
+            mask[(m0 + lane) * words + ((n0 + g) >> 5)] = word;
             vis += __popc(word);
         }
     }
+}
+
+template <bool CULL>
+__device__ void vis_item(const BatchParams& P, const DevScene& S, const GridView& G, int scene, int stage,
+                         long long n0, long long m0, int i0, int i1) {
+    const float* spos = stage == kVisBounce ? S.scat_pos : S.src_pos;
+    const long long ns = stage == kVisBounce ? S.n_scat : S.n_src;
+    const int* sid = stage == kVisBounce ? S.scat_id : nullptr;
+    const float* kpos = stage == kVisScat ? S.scat_pos : P.snk_pos;
+    const long long nk = stage == kVisScat ? S.n_scat : P.n_snk;
+    const int* kid = stage == kVisScat ? S.scat_id : P.snk_id;
+    const long long rem = ns - n0;
+    const int nsrc = (int)(rem < P.src_chunk ? rem : P.src_chunk);
+    unsigned int vis = 0, tests = 0;  // of one lane; diagnostic: wraps only past 2^32 tests
+    // The element stages turn the warp round: an array's elements see a sink along rays that cross the same cells (as in
+    // grid_transposed_kernel; 8 scenes of up to 3,969 elements, 16 frequencies: 64.0 -> 59.3 ms at (2, 64, 8), 57.1 ->
+    // 46.6 at (2, 32, 6)).  Scatter points as sources are turned for few sinks, which lie too far apart to share a walk
+    // (the rule of propagation.scatter_schedule), and where items are split.
+    if (stage != kVisBounce || P.turn_all)
+        vis_walks<CULL, true>(P, G, spos, sid, n0, nsrc, kpos, kid, m0, nk, i0, i1, S.mask[stage], S.mask_words[stage], vis, tests);
+    else
+        vis_walks<CULL, false>(P, G, spos, sid, n0, nsrc, kpos, kid, m0, nk, i0, i1, S.mask[stage], S.mask_words[stage], vis, tests);
     if (P.counters) {
-        const unsigned long long v = warp_sum(vis);
+        const unsigned long long v = warp_sum((unsigned long long)vis);
         const unsigned long long t = warp_sum((unsigned long long)tests);
-        if (lane == 0) {
+        if ((threadIdx.x & 31) == 0) {
             atomicAdd(P.counters + 4LL * scene + stage, v);
             atomicAdd(P.counters + 4LL * scene + 3, t);
         }
@@ -359,14 +376,11 @@ __device__ __forceinline__ void pair_freqs(const BatchParams& P, const PairCommo
 }
 
 // How the lanes of a warp set up the pairs of its sinks (field_item).  A pair's direction, distance, amplitude and
-// transverse excitation are the same at every frequency, and cost about as much as three frequencies: with more than
-// kAloneGroups frequency groups a sink, `per` pairs of each of the warp's sinks are set up at a time, a pair a lane, and
-// every lane of the sink then adds them at its own frequencies.  This lane sets up number `rank` of a sink whose bits
-// lane `at` holds, and reads those of its own sink from the lanes `from` .. `from` + per - 1.  With fewer groups each
-// lane sets up its own pairs (per = 1): no lane waits for another then.
-// 8 scenes, 1e8 pairs, one frequency a lane, 2 / 3 / 4 / 8 / 16 / 64 frequencies, each alone 27.5 / 28.9 / 31.4 / 33.3
-// / 56 / 134 ms, shared 36.4 / 36.7 / 31.6 / 28.9 / 29.8 / 35.5 ms.
-constexpr int kAloneGroups = 4;
+// transverse excitation are the same at every frequency, and cost about as much as three frequencies: `per` pairs of
+// each of the warp's sinks are set up at a time, a pair a lane, and every lane of the sink then adds them at its own
+// frequencies.  This lane sets up number `rank` of a sink whose bits lane `at` holds, and reads those of its own sink
+// from the lanes `from` .. `from` + per - 1.  8 scenes, 1e8 pairs, one frequency a lane, 8 / 16 / 64 frequencies: each
+// lane its own pairs 46 / 56 / 134 ms, shared 28.9 / 29.8 / 35.5 ms.
 struct Share {
     int per, rank, at, from;
     bool sets;
@@ -389,29 +403,20 @@ __device__ __forceinline__ void field_stage(const BatchParams& P, const unsigned
         float acc[6 * FG];
 #pragma unroll
         for (int k = 0; k < 6 * FG; ++k) acc[k] = 0.f;
-        if (sh.per == 1) {
-            while (bits) {
-                const int j = __ffs(bits) - 1;
-                bits &= bits - 1;
-                const PairCommon c = pair_common<FG, BOUNCE>(P, spos, src_E, (wi << 5) + j, ex, ey, ez, nx, ny, nz);
-                pair_freqs<FG, BOUNCE>(P, c, w, b0, f0, cnt, acc);
-            }
-        } else {
-            do {
-                unsigned int mine = __shfl_sync(full, bits, sh.at);  // without its `rank` lowest bits
-                for (int k = 0; k < sh.rank; ++k) mine &= mine - 1;
-                const int j = mine ? __ffs(mine) - 1 : 0;
-                if (sh.sets && mine)
-                    put_pair<BOUNCE>(ent, tid & 31, pair_common<FG, BOUNCE>(P, spos, src_E, (wi << 5) + j, ex, ey, ez, nx, ny, nz));
-                const int take = min(__popc(bits), sh.per);
-                __syncwarp();
-                for (int i = 0; i < take; ++i)
-                    pair_freqs<FG, BOUNCE>(P, get_pair<BOUNCE>(ent, sh.from + i), w, b0, f0, cnt, acc);
-                __syncwarp();
-                const int last = __shfl_sync(full, j, sh.from + max(take - 1, 0));
-                if (take) bits &= ~((2u << last) - 1u);
-            } while (__any_sync(full, bits != 0));
-        }
+        do {
+            unsigned int mine = __shfl_sync(full, bits, sh.at);  // without its `rank` lowest bits
+            for (int k = 0; k < sh.rank; ++k) mine &= mine - 1;
+            const int j = mine ? __ffs(mine) - 1 : 0;
+            if (sh.sets && mine)
+                put_pair<BOUNCE>(ent, tid & 31, pair_common<FG, BOUNCE>(P, spos, src_E, (wi << 5) + j, ex, ey, ez, nx, ny, nz));
+            const int take = min(__popc(bits), sh.per);
+            __syncwarp();
+            for (int i = 0; i < take; ++i)
+                pair_freqs<FG, BOUNCE>(P, get_pair<BOUNCE>(ent, sh.from + i), w, b0, f0, cnt, acc);
+            __syncwarp();
+            const int last = __shfl_sync(full, j, sh.from + max(take - 1, 0));
+            if (take) bits &= ~((2u << last) - 1u);
+        } while (__any_sync(full, bits != 0));
 #pragma unroll
         for (int k = 0; k < 6 * FG; ++k) sacc[k * kBT + tid] += acc[k];
     }
@@ -440,14 +445,13 @@ __device__ void field_item(const BatchParams& P, const DevScene& S, int scene, i
     sh.sets = own < sinks && m0 + own < nk;
     sh.at = sh.sets ? max(own * G - g0, 0) : lane;
     sh.from = ((int)ms - m0) * sh.per;
-    if (G <= kAloneGroups) sh.per = 1;  // (the warp may hold up to 32 sinks)
-    const long long ks = sh.per == 1 ? ms : (long long)m0 + own;
+    const long long ks = (long long)m0 + own;  // the sink whose pairs this lane sets up
 #pragma unroll
     for (int k = 0; k < 6 * FG; ++k) sacc[k * kBT + tid] = 0.f;
     float ex = 0.f, ey = 0.f, ez = 0.f, nx = 0.f, ny = 0.f, nz = 0.f;
     float2 b0 = make_float2(0.f, 0.f);
     if (ok) b0 = __ldg(P.beta_ff + f0);
-    if (sh.per == 1 ? ok : sh.sets) {
+    if (sh.sets) {
         const float* kp = (at_sinks ? P.snk_pos : S.scat_pos) + 3 * ks;
         const float* kn = (at_sinks ? P.snk_nrm : S.scat_nrm) + 3 * ks;
         ex = __ldg(kp); ey = __ldg(kp + 1); ez = __ldg(kp + 2);
@@ -479,6 +483,112 @@ __device__ void field_item(const BatchParams& P, const DevScene& S, int scene, i
             float* out = P.field + (((long long)scene * P.n_freq + f0 + j) * P.n_snk + m) * 6;
 #pragma unroll
             for (int k = 0; k < 6; ++k) out[k] = sacc[(6 * j + k) * kBT + tid];
+        }
+    }
+}
+
+// Few frequency groups (kPointGroups at most): a warp takes one point, its lanes a slice of the point's visible sources
+// for one group each, every lane with its own pairs; the slices are added at the end.  With a point and group a lane,
+// a sink's sources stand one behind the other on one lane, milliseconds for a few thousand of them, while most of the
+// chip has nothing to do.  8 scenes, 1e8 pairs, 1 / 4 frequencies (one a lane) 27.4 / 30.2 -> 20.4 / 22.3 ms, 16
+// frequencies (four a lane) 41 -> 25.6; 32 frequencies (four a lane, 8 groups) 38.4 -> 32.1; with 16 groups 27.9 -> 33.3.
+constexpr int kPointGroups = 8;
+
+// Adds the pairs of one stage: the visible sources' indices are listed (list: 64 ints of the warp) and taken L at a time,
+// 16 times in registers, then added to the thread's accumulator (sums in two levels, as in field_stage: one running sum
+// of a sink's thousands of pairs was 3 times further off).
+template <int FG, bool BOUNCE>
+__device__ __forceinline__ void point_stage(const BatchParams& P, const unsigned int* row, long long words,
+                                            const float* spos, const float* src_E, const float* w, float ex, float ey,
+                                            float ez, float nx, float ny, float nz, float2 b0, int f0, int cnt, int L,
+                                            int slice, int* list, float* sacc) {
+    const unsigned full = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const unsigned below = (1u << lane) - 1u;
+    int held = 0, rounds = 0;
+    float acc[6 * FG];
+#pragma unroll
+    for (int k = 0; k < 6 * FG; ++k) acc[k] = 0.f;
+    auto flush = [&]() {
+#pragma unroll
+        for (int k = 0; k < 6 * FG; ++k) {
+            sacc[k * kBT + tid] += acc[k];
+            acc[k] = 0.f;
+        }
+    };
+    auto add = [&](int count) {
+        if (slice < count) {
+            const PairCommon c = pair_common<FG, BOUNCE>(P, spos, src_E, list[slice], ex, ey, ez, nx, ny, nz);
+            pair_freqs<FG, BOUNCE>(P, c, w, b0, f0, cnt, acc);
+        }
+    };
+    for (long long w0 = 0; w0 < words; w0 += 32) {
+        const unsigned mine = w0 + lane < words ? row[w0 + lane] : 0u;
+        unsigned any = __ballot_sync(full, mine != 0);
+        while (any) {
+            const int k = __ffs(any) - 1;
+            any &= any - 1;
+            const unsigned bits = __shfl_sync(full, mine, k);
+            if ((bits >> lane) & 1u) list[held + __popc(bits & below)] = (int)((w0 + k) << 5) + lane;
+            held += __popc(bits);
+            __syncwarp();
+            while (held >= L) {
+                add(L);
+                if ((++rounds & 15) == 0) flush();
+                const int next = lane < held - L ? list[L + lane] : 0;
+                __syncwarp();
+                list[lane] = next;
+                held -= L;
+                __syncwarp();
+            }
+        }
+    }
+    add(held);
+    flush();
+    __syncwarp();
+}
+
+template <int FG>
+__device__ void point_item(const BatchParams& P, const DevScene& S, int scene, int kind, long long point, int* list,
+                           float* sacc) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool at_sinks = kind == kFieldE;
+    const int G = P.n_groups;
+    const int L = G == 1 ? 32 : G == 2 ? 16 : G <= 4 ? 8 : 4;  // slices, a power of two with G L <= 32
+    const int slice = lane / G < L ? lane / G : 64;  // (64: a lane left over)
+    const int g = lane % G;
+    const int f0 = g * FG;
+    const int cnt = min(FG, P.n_freq - f0);
+    const float* kp = (at_sinks ? P.snk_pos : S.scat_pos) + 3 * point;
+    const float* kn = (at_sinks ? P.snk_nrm : S.scat_nrm) + 3 * point;
+    const float ex = __ldg(kp), ey = __ldg(kp + 1), ez = __ldg(kp + 2);
+    const float nx = __ldg(kn), ny = __ldg(kn + 1), nz = __ldg(kn + 2);
+    const float2 b0 = __ldg(P.beta_ff + f0);
+#pragma unroll
+    for (int k = 0; k < 6 * FG; ++k) sacc[k * kBT + threadIdx.x] = 0.f;
+    const int vis = at_sinks ? kVisDirect : kVisScat;
+    point_stage<FG, false>(P, S.mask[vis] + point * S.mask_words[vis], S.mask_words[vis], S.src_pos, S.src_E, nullptr, ex,
+                           ey, ez, nx, ny, nz, b0, f0, cnt, L, slice, list, sacc);
+    if (at_sinks && S.n_scat > 0)
+        point_stage<FG, true>(P, S.mask[kVisBounce] + point * S.mask_words[kVisBounce], S.mask_words[kVisBounce],
+                              S.scat_pos, nullptr, S.w, ex, ey, ez, nx, ny, nz, b0, f0, cnt, L, slice, list, sacc);
+    float acc[6 * FG];
+#pragma unroll
+    for (int k = 0; k < 6 * FG; ++k) acc[k] = sacc[k * kBT + threadIdx.x];
+    for (int o = L / 2; o > 0; o /= 2) {
+#pragma unroll
+        for (int k = 0; k < 6 * FG; ++k) acc[k] += __shfl_down_sync(full, acc[k], o * G);
+    }
+    if (slice == 0) {
+        const long long m = !at_sinks ? point : P.snk_id ? (long long)__ldg(P.snk_id + point) : point;
+#pragma unroll
+        for (int j = 0; j < FG; ++j) {
+            if (j >= cnt) break;
+            float* out = at_sinks ? P.field + (((long long)scene * P.n_freq + f0 + j) * P.n_snk + m) * 6
+                                  : S.w + (point * P.n_freq + f0 + j) * 6;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) out[k] = acc[6 * j + k];
         }
     }
 }
@@ -539,13 +649,15 @@ __global__ void __launch_bounds__(kBT, MINB) batch_kernel(const BatchParams P) {
             if (kind < kFieldW)
                 vis_item<CULL>(P, S, s_grid[wid], scene, kind, (long long)a, (long long)b,
                                part * (kWarpSinks / P.split), (part + 1) * (kWarpSinks / P.split));
+            else if (P.n_groups <= kPointGroups)
+                for (int t = 0; t < b; ++t)  // b consecutive points
+                    point_item<FG>(P, S, scene, kind, (long long)a + t, reinterpret_cast<int*>(s_ent[wid]), sacc);
             else
                 for (int t = 0; t < b; ++t)  // b consecutive 32-slot chunks
                     field_item<FG>(P, S, scene, kind, (long long)a + t, s_ent[wid], sacc);
         }
-        __threadfence();
         __syncwarp();
-        if (lane == 0) atomicAdd(P.done + (long long)scene * kKinds + kind, 1u);
+        if (lane == 0) add_release(P.done + (long long)scene * kKinds + kind, 1u);
     }
 }
 
@@ -643,9 +755,9 @@ int make_plan(const lyem_batch_scene* sc, int n_scenes, long long n_snk, int n_f
     // A field item is a run of 32-slot chunks (slot = point * groups + group),
     // long enough for about kItemPairs candidate (pair, group) evaluations.
     // The list holds its parts: a chunk each (more where a point has fewer
-    // than 64 sources), since a warp adds a chunk's pairs one behind the other
-    // whatever the number of groups, and long runs left most warps without
-    // work.  8 scenes of up to 178 elements, 1,649 sinks, 8 / 64 frequencies:
+    // than 64 sources), or a point each (more where it has fewer than 512),
+    // since a warp adds their pairs one behind the other whatever the number
+    // of groups, and long runs left most warps without work.  8 scenes of up to 178 elements, 1,649 sinks, 8 / 64 frequencies:
     // whole items 9.0 / 25.8 ms, parts 3.4 / 4.4 ms; 8 of up to 4,096, 4,000
     // sinks, 16 / 64 frequencies: 35.6 / 72.8 and 29.8 / 35.3 ms.
     auto add_field = [&](int s, int kind, long long nk, long long pairs_per_sink) {
@@ -653,10 +765,12 @@ int make_plan(const lyem_batch_scene* sc, int n_scenes, long long n_snk, int n_f
         const long long per_chunk = std::max(1LL, pairs_per_sink * 32 / groups);
         const long long k = std::min(64LL, std::max(1LL, (kItemPairs + per_chunk - 1) / per_chunk));
         pl.count[kind] += (chunks + k - 1) / k;
-        const long long part = std::max(1LL, 64 / std::max(1LL, pairs_per_sink));
-        for (long long c = 0; c < chunks; c += part)
-            pl.items.push_back(make_int4(kind, s, (int)c, (int)std::min(part, chunks - c)));
-        pl.expect[(size_t)s * kKinds + kind] = (int)((chunks + part - 1) / part);
+        const bool by_point = groups <= kPointGroups;  // (point_item: the chunk is a point)
+        const long long n = by_point ? nk : chunks;
+        const long long part = std::max(1LL, (by_point ? 512 : 64) / std::max(1LL, pairs_per_sink));
+        for (long long c = 0; c < n; c += part)
+            pl.items.push_back(make_int4(kind, s, (int)c, (int)std::min(part, n - c)));
+        pl.expect[(size_t)s * kKinds + kind] = (int)((n + part - 1) / part);
     };
     for (int s : order) add_field(s, kFieldW, sc[s].n_scat, sc[s].n_src);
     for (int s : order) add_field(s, kFieldE, n_snk, sc[s].n_src + sc[s].n_scat);

@@ -35,17 +35,18 @@ C0 = 299792458.0
 # (frequencies per thread, sources per visibility item, blocks per SM).  Blocks per
 # SM 3, 4, 6 or 8 select kernel variants whose registers are capped for that
 # occupancy; 0 runs the uncapped variant with as many blocks as fit.
-CANDIDATES = [(1, 32, 8), (1, 32, 4), (1, 64, 8), (1, 64, 4), (2, 32, 6), (2, 32, 4), (4, 32, 4)]
+CANDIDATES = [(1, 32, 4), (1, 32, 8), (1, 64, 4), (2, 32, 4), (4, 32, 4), (4, 32, 3), (4, 64, 4), (8, 32, 3)]
 
 
-def default_config(n_freq):
-    """Configuration of a batch that is not tuned: one frequency per thread (the threads of a sink share the set-up of its
-    pairs), with the most warps for the walks up to four frequencies and the most registers for the fields from there on.
-    Milliseconds at (1, 32, 8) / (1, 32, 4) / (2, 32, 6) / (4, 32, 4): 8 scenes, 1e8 pairs, 1 frequency 26.4 / 27.5 / 28.3
-    / 30.3, 4 frequencies 31.4 / 30.2 / 31.0 / 34.1, 16 frequencies 33.8 / 29.9 / 33.4 / 39.8, 64 frequencies 43.9 / 35.3
-    / 38.9 / 46.8; 8 scenes, 8e6 pairs, 1 frequency 2.8 / 2.9 / 3.4 / 3.3, 4 frequencies 2.9 / 3.1 / 3.7 / 3.9, 16
-    frequencies 3.9 / 3.8 / 4.6 / 4.3, 64 frequencies 5.4 / 4.4 / 5.6 / 6.3."""
-    return (1, 32, 8) if n_freq <= 4 else (1, 32, 4)
+def default_config(n_freq, uniform):
+    """Configuration of a batch that is not tuned.  3 to 16 uniform frequencies: four per thread, at most four groups of
+    them a sink, whose threads share its sources; otherwise one per thread (many groups share the set-up of a pair instead,
+    and do not need the rotation).  Milliseconds at (1, 32, 8) / (1, 32, 4) / (2, 32, 4) / (4, 32, 4): 8 scenes, 1e8 pairs,
+    1 frequency 22.4 / 20.5 / 21.0 / 21.0, 4 frequencies 24.9 / 22.1 / 21.7 / 21.5, 16 frequencies 31.0 / 27.9 / 28.7 /
+    25.7, 17 frequencies (four a thread are five groups) - / 30.8 / 32.5 / 32.2, 64 frequencies - / 34.5 / 34.8 / 42.8; 8
+    scenes, 8e6 pairs, 1 frequency 1.9 / 2.0 / 2.0 / 2.1, 4 frequencies 2.4 / 2.2 / 2.2 / 2.2, 16 frequencies 3.6 / 3.4 /
+    3.2 / 3.0, 64 frequencies - / 4.2 / 4.5 / 5.7."""
+    return (4, 32, 4) if uniform and 3 <= n_freq <= 16 else (1, 32, 4)
 
 
 def stratified_subset(scenes, n_sinks, every=4):
@@ -202,7 +203,7 @@ class BatchedScattering:
     # ------------------------------------------------------------ configuration
 
     def _default(self):
-        return default_config(self.n_freq)
+        return default_config(self.n_freq, self.uniform)
 
     def _cfg(self, c):
         cfg = BatchConfig()

@@ -239,11 +239,12 @@ def test_split_visibility_items(copies, n_snk):
     assert st == 0 and flags == 0
 
 
-@pytest.mark.parametrize("fg,n_freq", [(1, 1), (1, 4), (1, 5), (1, 17), (1, 31), (1, 32), (1, 33), (1, 65), (2, 8), (2, 9),
-                                       (2, 61), (4, 24), (8, 41)])
+@pytest.mark.parametrize("fg,n_freq", [(1, 1), (1, 2), (1, 3), (1, 4), (1, 5), (1, 8), (1, 9), (1, 17), (1, 31), (1, 32),
+                                       (1, 33), (1, 65), (2, 8), (2, 9), (2, 17), (2, 61), (4, 16), (4, 24), (8, 41)])
 def test_shared_pair_setup(fg, n_freq):
-    """Frequency groups on both sides of the line from which the lanes of a sink share its pairs' set-up, and that split
-    a warp between sinks unevenly: first, middle and last frequency against the per-scene pair stages."""
+    """Frequency groups on both sides of the line from which the lanes of a sink share its pairs' set-up instead of its
+    sources, and that split a warp between slices or sinks unevenly: first, middle and last frequency against the
+    per-scene pair stages."""
     B, P, SC = _mods()
     scenes, snk, snk_n = _small_batch(n_snk=83)
     freqs = np.linspace(25e9, 29e9, n_freq) if n_freq > 1 else np.array([27e9])

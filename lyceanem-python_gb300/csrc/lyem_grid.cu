@@ -458,82 +458,118 @@ __device__ __forceinline__ float tri_centroid(float4 v0, float4 e1, float4 e2, i
     return a[k] + (e[k] + f[k]) * (1.f / 3.f);
 }
 
+// A warp per cell.  Split: of the planes at k/8 of the cell (k = 1..7) on each axis, the one with the least surface-area
+// cost (the clipped child boxes' areas times their triangle counts, a ray's chance of entering a box being about
+// proportional to its area), a plane a lane; a triangle goes to child A when its centroid lies below the plane.
+// Visibility does not depend on the split.  Then a triangle a lane, in order.  With a thread per cell that tried the 21
+// planes one after the other, the launch lasted as long as its fullest cell: a whole grid
+// of 120,000 triangles in 21,853 cells 0.92 -> 0.26 ms, in 788,298 cells 0.70 -> 0.69, of 1,120,000 in 339,488 2.9 -> 1.2.
 __global__ void cell_fill_kernel(BinSpec b, const float4* __restrict__ tris, const int* __restrict__ vals,
                                  const int* __restrict__ cell_start, long long ncells, float4* __restrict__ cell_tris,
                                  float4* __restrict__ box) {
-    const long long plane = (long long)b.dims[0] * b.dims[1];
-    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < ncells;
-         c += (long long)gridDim.x * blockDim.x) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const long long plane_cells = (long long)b.dims[0] * b.dims[1];
+    const long long warps = (long long)gridDim.x * blockDim.x / 32;
+    for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32; c < ncells; c += warps) {
         const int q0 = cell_start[c], q1 = cell_start[c + 1];
-        const long long iz = c / plane, rem = c - iz * plane, iy = rem / b.dims[0], ix = rem - iy * b.dims[0];
+        const long long iz = c / plane_cells, rem = c - iz * plane_cells, iy = rem / b.dims[0], ix = rem - iy * b.dims[0];
         const float ci[3] = {(float)ix, (float)iy, (float)iz};
-        // split: of the planes at k/8 of the cell (k = 1..7) on each axis, the one
-        // with the least surface-area cost (the clipped child boxes' areas times
-        // their triangle counts, a ray's chance of entering a box being about
-        // proportional to its area); a triangle goes to child A when its centroid
-        // lies below the plane.  Visibility does not depend on the split.
+        float loA[3], hiA[3], loB[3], hiB[3];
+        auto reset = [&]() {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                loA[k] = loB[k] = INFINITY;
+                hiA[k] = hiB[k] = -INFINITY;
+            }
+        };
+        auto clipped_area = [&](const float* lo, const float* hi) {
+            float ext[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const float c0 = b.org[d] + ci[d] * b.cell;
+                ext[d] = fmaxf(fminf(hi[d], c0 + b.cell + 2.f * b.pad) - fmaxf(lo[d], c0 - 2.f * b.pad), 0.f);
+            }
+            return ext[0] * ext[1] + ext[1] * ext[2] + ext[2] * ext[0];
+        };
         int ax = 0;
         float mid = b.org[0] + (ci[0] + 0.5f) * b.cell;
         if (q1 - q0 > 1) {
-            float best = INFINITY;
-            for (int a = 0; a < 3; ++a) {
-                for (int k = 1; k < 8; ++k) {
-                    const float plane = b.org[a] + (ci[a] + 0.125f * (float)k) * b.cell;
-                    float lo[2][3], hi[2][3];
-                    int n[2] = {0, 0};
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) {
-                            lo[h][d] = INFINITY;
-                            hi[h][d] = -INFINITY;
-                        }
-                    for (int r = q0; r < q1; ++r) {
-                        const float4* t = tris + 3 * (long long)vals[r];
-                        const float4 v0 = t[0], e1 = t[1], e2 = t[2];
-                        const int h = tri_centroid(v0, e1, e2, a) < plane ? 0 : 1;
-                        ++n[h];
-                        tri_box(b, v0, e1, e2, lo[h], hi[h]);
-                    }
-                    float cost = 0.f;
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        if (!n[h]) continue;
-                        float ext[3];
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) {
-                            const float c0 = b.org[d] + ci[d] * b.cell;
-                            ext[d] = fmaxf(fminf(hi[h][d], c0 + b.cell + 2.f * b.pad) -
-                                               fmaxf(lo[h][d], c0 - 2.f * b.pad), 0.f);
-                        }
-                        cost += (ext[0] * ext[1] + ext[1] * ext[2] + ext[2] * ext[0]) * (float)n[h];
-                    }
-                    if (cost < best) {
-                        best = cost;
-                        ax = a;
-                        mid = plane;
-                    }
+            const int a = min(lane / 7, 2), k = lane % 7 + 1;
+            const float oa = a == 0 ? b.org[0] : a == 1 ? b.org[1] : b.org[2];
+            const float plane = oa + ((a == 0 ? ci[0] : a == 1 ? ci[1] : ci[2]) + 0.125f * (float)k) * b.cell;
+            int nA = 0, nB = 0;
+            reset();
+            for (int r = q0; r < q1; ++r) {
+                const float4* t = tris + 3 * (long long)vals[r];
+                const float4 v0 = t[0], e1 = t[1], e2 = t[2];
+                const float cen = a == 0 ? tri_centroid(v0, e1, e2, 0) : a == 1 ? tri_centroid(v0, e1, e2, 1)
+                                                                                : tri_centroid(v0, e1, e2, 2);
+                if (cen < plane) {
+                    ++nA;
+                    tri_box(b, v0, e1, e2, loA, hiA);
+                } else {
+                    ++nB;
+                    tri_box(b, v0, e1, e2, loB, hiB);
                 }
+            }
+            float cost = 0.f;
+            if (nA) cost += clipped_area(loA, hiA) * (float)nA;
+            if (nB) cost += clipped_area(loB, hiB) * (float)nB;
+            // the first of the planes of least cost (costs are not negative; the middle of x if none is finite)
+            const unsigned key = lane < 21 && cost < INFINITY ? __float_as_uint(cost) : 0xffffffffu;
+            const unsigned least = __reduce_min_sync(full, key);
+            if (least != 0xffffffffu) {
+                const int best = __ffs(__ballot_sync(full, key == least)) - 1;
+                ax = best / 7;
+                mid = __shfl_sync(full, plane, best);
             }
         }
         int na = 0;
-        for (int r = q0; r < q1; ++r) {
-            const float4* t = tris + 3 * (long long)vals[r];
-            na += tri_centroid(t[0], t[1], t[2], ax) < mid ? 1 : 0;
+        for (int r0 = q0; r0 < q1; r0 += 32) {
+            bool in_a = false;
+            if (r0 + lane < q1) {
+                const float4* t = tris + 3 * (long long)vals[r0 + lane];
+                in_a = tri_centroid(t[0], t[1], t[2], ax) < mid;
+            }
+            na += __popc(__ballot_sync(full, in_a));
         }
-        float loA[3] = {INFINITY, INFINITY, INFINITY}, hiA[3] = {-INFINITY, -INFINITY, -INFINITY};
-        float loB[3] = {INFINITY, INFINITY, INFINITY}, hiB[3] = {-INFINITY, -INFINITY, -INFINITY};
+        reset();
         int ia = q0, ib = q0 + na;
-        for (int r = q0; r < q1; ++r) {
-            const float4* t = tris + 3 * (long long)vals[r];
-            const float4 v0 = t[0], e1 = t[1], e2 = t[2];
-            const bool in_a = tri_centroid(v0, e1, e2, ax) < mid;
-            const int o = in_a ? ia++ : ib++;
-            cell_tris[3 * (long long)o] = v0;
-            cell_tris[3 * (long long)o + 1] = e1;
-            cell_tris[3 * (long long)o + 2] = e2;
-            if (in_a) tri_box(b, v0, e1, e2, loA, hiA);
-            else tri_box(b, v0, e1, e2, loB, hiB);
+        for (int r0 = q0; r0 < q1; r0 += 32) {
+            const bool ok = r0 + lane < q1;
+            float4 v0, e1, e2;
+            bool in_a = false;
+            if (ok) {
+                const float4* t = tris + 3 * (long long)vals[r0 + lane];
+                v0 = t[0];
+                e1 = t[1];
+                e2 = t[2];
+                in_a = tri_centroid(v0, e1, e2, ax) < mid;
+            }
+            const unsigned ma = __ballot_sync(full, in_a), mb = __ballot_sync(full, ok && !in_a);
+            if (ok) {
+                const int o = in_a ? ia + __popc(ma & below) : ib + __popc(mb & below);
+                cell_tris[3 * (long long)o] = v0;
+                cell_tris[3 * (long long)o + 1] = e1;
+                cell_tris[3 * (long long)o + 2] = e2;
+                if (in_a) tri_box(b, v0, e1, e2, loA, hiA);
+                else tri_box(b, v0, e1, e2, loB, hiB);
+            }
+            ia += __popc(ma);
+            ib += __popc(mb);
+        }
+        if (q1 > q0) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    loA[k] = fminf(loA[k], __shfl_xor_sync(full, loA[k], o));
+                    hiA[k] = fmaxf(hiA[k], __shfl_xor_sync(full, hiA[k], o));
+                    loB[k] = fminf(loB[k], __shfl_xor_sync(full, loB[k], o));
+                    hiB[k] = fmaxf(hiB[k], __shfl_xor_sync(full, hiB[k], o));
+                }
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -544,11 +580,13 @@ __global__ void cell_fill_kernel(BinSpec b, const float4* __restrict__ tris, con
             loB[k] = fmaxf(loB[k], clo);
             hiB[k] = fminf(hiB[k], chi);
         }
-        const int qm = q0 + na;
-        box[4 * c] = make_float4(loA[0], loA[1], loA[2], __int_as_float(q0));
-        box[4 * c + 1] = make_float4(hiA[0], hiA[1], hiA[2], __int_as_float(qm));
-        box[4 * c + 2] = make_float4(loB[0], loB[1], loB[2], __int_as_float(qm));
-        box[4 * c + 3] = make_float4(hiB[0], hiB[1], hiB[2], __int_as_float(q1));
+        if (lane == 0) {
+            const int qm = q0 + na;
+            box[4 * c] = make_float4(loA[0], loA[1], loA[2], __int_as_float(q0));
+            box[4 * c + 1] = make_float4(hiA[0], hiA[1], hiA[2], __int_as_float(qm));
+            box[4 * c + 2] = make_float4(loB[0], loB[1], loB[2], __int_as_float(qm));
+            box[4 * c + 3] = make_float4(hiB[0], hiB[1], hiB[2], __int_as_float(q1));
+        }
     }
 }
 
@@ -769,7 +807,7 @@ cudaError_t grid_fill(const BinSpec& b, const float4* tris, long long n_tris, co
     if (e != cudaSuccess) return e;
     const long long ncells = (long long)b.dims[0] * b.dims[1] * b.dims[2];
     if (cell_box) {
-        cell_fill_kernel<<<grid_blocks(ncells, 128), 128, 0, stream>>>(b, tris, vals, cell_start, ncells, cell_tris,
+        cell_fill_kernel<<<grid_blocks(32 * ncells, 128), 128, 0, stream>>>(b, tris, vals, cell_start, ncells, cell_tris,
                                                                       cell_box);
         note_launches(1);
     } else if (n_refs > 0) {

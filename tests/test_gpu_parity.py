@@ -861,3 +861,42 @@ def test_scene_cache_reuses_device_grid():
     FD.calculate_scattering(ap, sk, Mesh(v2, [("triangle", f)]), axis, beta=150.0, cuda=True)
     assert A.cache_stats["misses"] == m0 + 2
     _no_device_errors()
+
+
+@pytest.mark.parametrize("count", [1, 2, 31, 32, 33, 64, 65, 200])
+def test_cell_table_of_full_cells(count):
+    """A cell with fewer, as many and more triangles than a warp has lanes: its children hold its triangles, each once and
+    in triangle order, A's centroids below one of the 21 planes and B's above, each box its triangles' padded boxes."""
+    from lyceanem_gb300 import propagation as P
+    rng = np.random.default_rng(count)
+    cen = rng.uniform(0.2, 0.8, (count, 1, 3))
+    v = (cen + rng.uniform(-0.02, 0.02, (count, 3, 3))).astype(np.float32)
+    far = np.array([[[5.5, 5.5, 5.5], [5.6, 5.5, 5.5], [5.5, 5.6, 5.5]]], np.float32)
+    verts = np.concatenate([v, far]).reshape(-1, 3)
+    tris = P.pack_triangles(torch.from_numpy(verts), torch.arange(3 * (count + 1), dtype=torch.int32).reshape(-1, 3))
+    g = P.UniformGrid(tris, cell=6.0)
+    start, box = g.cell_start.cpu().numpy(), g.cell_box.cpu().numpy()
+    refs = np.ascontiguousarray(box[:, [3, 7, 11, 15]]).view(np.int32)
+    c = int(np.argmax(np.diff(start)))
+    q0, q1 = start[c], start[c + 1]
+    packed = tris.cpu().numpy()
+    got = g.cell_tris.cpu().numpy()[q0:q1]
+    index = {row.tobytes(): k for k, row in enumerate(packed)}
+    ids = [index[row.tobytes()] for row in got]
+    na = refs[c, 1] - q0
+    assert tuple(refs[c]) == (q0, q0 + na, q0 + na, q1) and q1 - q0 >= count and len(set(ids)) == len(ids)
+    A, B = ids[:na], ids[na:]
+    assert A == sorted(A) and B == sorted(B)
+    p = verts.reshape(-1, 3, 3)
+    if len(ids) > 1 and A and B:
+        m = p.astype(np.float64).mean(1)
+        planes = [(a, g.origin[a] + (0.125 * k + (c // [1, g.dims[0], g.dims[0] * g.dims[1]][a]) % g.dims[a]) * g.cell)
+                  for a in range(3) for k in range(1, 8)]
+        assert any((m[A, a] < x + 1e-5).all() and (m[B, a] > x - 1e-5).all() for a, x in planes)
+    pad = 1e-3 * g.cell
+    for child, lo, hi in ((A, box[c, 0:3], box[c, 4:7]), (B, box[c, 8:11], box[c, 12:15])):
+        if child:  # (a vertex is formed as v0 + edge in FP32: an ulp of 6 m is 5e-7)
+            assert np.allclose(lo, p[child].min((0, 1)) - pad, atol=2e-6)
+            assert np.allclose(hi, p[child].max((0, 1)) + pad, atol=2e-6)
+    if count > 2:
+        assert na > 0

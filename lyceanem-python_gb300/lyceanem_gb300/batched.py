@@ -35,7 +35,7 @@ C0 = 299792458.0
 # (frequencies per thread, sources per visibility item, blocks per SM).  Blocks per
 # SM 3, 4, 6 or 8 select kernel variants whose registers are capped for that
 # occupancy; 0 runs the uncapped variant with as many blocks as fit.
-CANDIDATES = [(1, 32, 4), (1, 32, 8), (1, 64, 4), (2, 32, 4), (4, 32, 4), (4, 32, 3), (4, 64, 4), (8, 32, 3)]
+CANDIDATES = [(1, 32, 4), (1, 32, 8), (1, 64, 4), (2, 64, 6), (2, 32, 6), (2, 32, 4), (4, 32, 4), (4, 64, 4), (8, 32, 3)]
 
 
 def default_config(n_freq, uniform):

@@ -510,11 +510,9 @@ def run_sweep(args, n_check=256, reps=5):
     peak, peak_src = measured_peak("bf16_tflops")
     res["tensor_issued_flops"] = issued
     outs = {}
-    for name, mode, k_tile, mc in (("fp32", "fp32", 32, False), ("bf16x3g", "bf16x3g", 32, False),
-                                   ("fp16x3g", "fp16x3g", 32, False), ("bf16x3g_k64", "bf16x3g", 64, False),
-                                   ("bf16x3g_multicast", "bf16x3g", 32, True)):
+    for name, mode, k_tile in (("fp32", "fp32", 32), ("bf16x3g", "bf16x3g", 32), ("fp16x3g", "fp16x3g", 32),
+                               ("bf16x3g_k64", "bf16x3g", 64)):
         BS.set_k_tile(k_tile)
-        BS.set_multicast(mc)
         sw = BS.BeamSweep(G, mode)
         torch.cuda.synchronize()
         px, py = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -537,13 +535,11 @@ def run_sweep(args, n_check=256, reps=5):
                      "prepare_network_ms": px.elapsed_time(py)}
         if mode != "fp32":
             res[name]["k_tile"] = k_tile
-            res[name]["multicast_clusters"] = mc
             res[name]["tensor_tflops_issued"] = issued / (ms * 1e-3) / 1e12
             res[name]["tensor_frac"] = issued / (ms * 1e-3) / 1e12 / peak
         del sw, out
         torch.cuda.empty_cache()
     BS.set_k_tile(32)
-    BS.set_multicast(False)
     st, flags = P.device_errors()
     res["device_errors"] = [int(st), int(flags)]
     res["roofline"] = {"bound": "tensor", "kernel": "sweep_tc_kernel (bf16x3g, k-tile 32, single-CTA)",

@@ -239,8 +239,7 @@ LYEM_API int lyem_sweep_set_k_tile(int32_t k_tile) {
 
 LYEM_API int lyem_sweep_set_multicast(int32_t on) {
     if (on != 0 && on != 1) return LYEM_ERR_INVALID;
-    sweep_tc_multicast = on;
-    return LYEM_OK;
+    return LYEM_OK;  // there is one tensor-core kernel
 }
 
 LYEM_API int lyem_sweep_prepare_network(const float* d_pairs, int64_t n_src, int64_t n_snk, int32_t mode, int64_t ld,

@@ -70,12 +70,7 @@ struct TcParams {
     unsigned int* err;       // device error word
 };
 
-// MC: CTAs run in clusters of two that take the row tiles 2 i and 2 i + 1 of one
-// beam tile; each loads half of the shared weight tile and multicasts it to both,
-// so each SM requests 2/3 of the operand bytes of a stage, and a stage is
-// refilled only after both CTAs' MMAs have read it (its empty barrier counts an
-// arrival from each).
-template <int BK, int BN, bool BF16, bool MC>
+template <int BK, int BN, bool BF16>
 __global__ void __launch_bounds__(kTcThreads, 1)
     sweep_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const TcParams p) {
@@ -96,7 +91,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kStages; ++s) {
             mbar_init(bar(FULL + s), 1);
-            mbar_init(bar(EMPTY + s), MC ? 2 : 1);
+            mbar_init(bar(EMPTY + s), 1);
         }
         mbar_init(bar(MID_FULL), 1);
         mbar_init(bar(MID_DONE), 4);
@@ -109,25 +104,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     if (warp == 1) tc::tmem_alloc(smem_addr(s_tmem), kTmemCols);
     tc::fence_before();
-    if (MC)
-        tc::cluster_sync();  // the peer's multicast copies and commits may target these barriers from now on
-    else
-        __syncthreads();
+    __syncthreads();
     tc::fence_after();
     const uint32_t tmem = *s_tmem;
-    // tile t -> (component, row tile, beam tile); with MC a cluster takes tile t and the CTA of rank r its row
-    // tile 2 mt + r (past the last row tile for an odd count: zero rows, nothing stored)
-    const int rank = MC ? (int)tc::cluster_ctarank() : 0;
-    const int first = MC ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-    const int step = MC ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-    const int n_rt = MC ? (p.n_mt + 1) / 2 : p.n_mt;
-    const int tiles = 3 * n_rt * p.n_kt;
+    // tile t -> (component, row tile, beam tile)
+    const int first = (int)blockIdx.x, step = (int)gridDim.x;
+    const int tiles = 3 * p.n_mt * p.n_kt;
     auto decode = [&](int t, int& c, int& mt, int& kt) {
-        c = t / (n_rt * p.n_kt);
-        const int rem = t - c * (n_rt * p.n_kt);
+        c = t / (p.n_mt * p.n_kt);
+        const int rem = t - c * (p.n_mt * p.n_kt);
         mt = rem / p.n_kt;
         kt = rem - mt * p.n_kt;
-        if (MC) mt = 2 * mt + rank;
     };
 
     // Bounded wait; gives up early once another role has given up.
@@ -176,16 +163,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         const int x = kb * BK, pa = (c * 3 + q) * 2;
                         tc::tma_load_3d(st, &tmA, x, mt * kBM, pa, fb);
                         tc::tma_load_3d(st + C::kABytes, &tmA, x, mt * kBM, pa + 1, fb);
-                        if (MC) {  // this CTA's half of the weight rows, into both CTAs
-                            const uint32_t half = (uint32_t)rank * (C::kBBytes / 2);
-                            const int y = kt * BN + rank * (BN / 2);
-                            tc::tma_load_3d_mc(st + 2 * C::kABytes + half, &tmB, x, y, 2 * q, fb, 0x3);
-                            tc::tma_load_3d_mc(st + 2 * C::kABytes + C::kBBytes + half, &tmB, x, y, 2 * q + 1, fb,
-                                               0x3);
-                        } else {
-                            tc::tma_load_3d(st + 2 * C::kABytes, &tmB, x, kt * BN, 2 * q, fb);
-                            tc::tma_load_3d(st + 2 * C::kABytes + C::kBBytes, &tmB, x, kt * BN, 2 * q + 1, fb);
-                        }
+                        tc::tma_load_3d(st + 2 * C::kABytes, &tmB, x, kt * BN, 2 * q, fb);
+                        tc::tma_load_3d(st + 2 * C::kABytes + C::kBBytes, &tmB, x, kt * BN, 2 * q + 1, fb);
                         issued[s] = true;
                         last_par[s] = ph;
                         if (++s == C::kStages) {
@@ -236,11 +215,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                             tc::mma_f16_lastuse_a(acc, ah, bl, idesc, 1u);
                             tc::mma_f16(acc, al, bh, idesc, 1u);
                         }
-                        // the stage is free once these MMAs (and, with MC, the peer's) complete
-                        if (MC)
-                            tc::commit_mc(bar(EMPTY + s), 0x3);
-                        else
-                            tc::commit(bar(EMPTY + s));
+                        // the stage is free once these MMAs complete
+                        tc::commit(bar(EMPTY + s));
                         if (++s == C::kStages) {
                             s = 0;
                             ph ^= 1u;
@@ -319,10 +295,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
     }
     tc::fence_before();
-    if (MC)
-        tc::cluster_sync();  // neither CTA leaves while the other may still copy into or arrive on it
-    else
-        __syncthreads();
+    __syncthreads();
     if (warp == 1) {
         __syncwarp();  // dealloc is a .sync.aligned warp instruction
         tc::fence_after();
@@ -364,56 +337,24 @@ bool make_map(CUtensorMap* m, const void* base, bool bf16, int k, int rows, int 
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BK, int BN, bool BF16, bool MC>
-cudaError_t launch_tc(const CUtensorMap& a, const CUtensorMap& b, const TcParams& p, cudaStream_t stream,
-                      bool* launched) {
+template <int BK, int BN, bool BF16>
+cudaError_t launch_tc(const CUtensorMap& a, const CUtensorMap& b, const TcParams& p, cudaStream_t stream) {
     using C = TcCfg<BK, BN>;
-    auto kern = sweep_tc_kernel<BK, BN, BF16, MC>;
-    *launched = false;
+    auto kern = sweep_tc_kernel<BK, BN, BF16>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
     if (e != cudaSuccess) return e;
     const int sms = device_sm_count();
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(kTcThreads);
-    cfg.dynamicSmemBytes = C::kSmem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    if (MC) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        const int tiles = 3 * ((p.n_mt + 1) / 2) * p.n_kt;
-        cfg.gridDim = dim3(2 * sms);  // the occupancy query needs a grid shape
-        int clusters = 0;
-        e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
-        if (e != cudaSuccess || clusters < 1) {
-            (void)cudaGetLastError();
-            return cudaSuccess;  // no co-resident pair: the caller uses the single-CTA kernel
-        }
-        cfg.gridDim = dim3(2 * (unsigned)(tiles < clusters ? tiles : clusters));
-    } else {
-        const int tiles = 3 * p.n_mt * p.n_kt;
-        cfg.gridDim = dim3((unsigned)(tiles < sms ? tiles : sms));
-    }
-    e = cudaLaunchKernelEx(&cfg, kern, a, b, p);
-    if (e != cudaSuccess) return e;
-    *launched = true;
+    const int tiles = 3 * p.n_mt * p.n_kt;
+    kern<<<(unsigned)(tiles < sms ? tiles : sms), kTcThreads, C::kSmem, stream>>>(a, b, p);
     note_launches(1);
     return cudaGetLastError();
 }
 
 template <int BN>
-cudaError_t launch_single(int bk, bool bf16, const CUtensorMap& a, const CUtensorMap& b, const TcParams& p,
-                          cudaStream_t stream) {
-    bool done = false;
-    if (bk == 64)
-        return bf16 ? launch_tc<64, BN, true, false>(a, b, p, stream, &done)
-                    : launch_tc<64, BN, false, false>(a, b, p, stream, &done);
-    return bf16 ? launch_tc<32, BN, true, false>(a, b, p, stream, &done)
-                : launch_tc<32, BN, false, false>(a, b, p, stream, &done);
+cudaError_t launch_bn(int bk, bool bf16, const CUtensorMap& a, const CUtensorMap& b, const TcParams& p,
+                      cudaStream_t stream) {
+    if (bk == 64) return bf16 ? launch_tc<64, BN, true>(a, b, p, stream) : launch_tc<64, BN, false>(a, b, p, stream);
+    return bf16 ? launch_tc<32, BN, true>(a, b, p, stream) : launch_tc<32, BN, false>(a, b, p, stream);
 }
 
 // Beams per tile.  256 keeps the tensor pipe fullest; where its tiles leave SMs idle or are mostly padding, narrower ones
@@ -439,7 +380,6 @@ int tile_beams(long long row_tiles, long long n_beams) {
 }  // namespace
 
 int sweep_tc_k_tile = 32;
-int sweep_tc_multicast = 0;
 
 int launch_sweep_tc(const void* network, const void* weights, int64_t n_src, int64_t n_snk, int64_t ld,
                     int64_t n_beams, bool bf16, float* out, int64_t ldc, cudaStream_t stream) {
@@ -448,7 +388,7 @@ int launch_sweep_tc(const void* network, const void* weights, int64_t n_src, int
     const unsigned char* na = static_cast<const unsigned char*>(network);
     const unsigned char* wb = static_cast<const unsigned char*>(weights);
     const int n_mt = (int)((n_snk + kBM - 1) / kBM);
-    const int bn = sweep_tc_multicast ? 256 : tile_beams(n_mt, n_beams);
+    const int bn = tile_beams(n_mt, n_beams);
     CUtensorMap ma, mb;
     if (!make_map(&ma, na + kSweepHeaderBytes, bf16, (int)n_src, (int)n_snk, 18, kpad, ld, bk, kBM) ||
         !make_map(&mb, wb + kSweepHeaderBytes, bf16, (int)n_src, (int)n_beams, 6, kpad, n_beams, bk, bn))
@@ -466,23 +406,9 @@ int launch_sweep_tc(const void* network, const void* weights, int64_t n_src, int
     p.scale_w = reinterpret_cast<const float*>(wb);
     p.err = device_error_word();
     if (!p.err) return LYEM_ERR_CUDA;
-    cudaError_t e = cudaSuccess;
-    bool done = false;
-    if (sweep_tc_multicast) {  // clusters of two sharing the weight tile; the single-CTA kernel if none fit
-        CUtensorMap mb_half;
-        if (!make_map(&mb_half, wb + kSweepHeaderBytes, bf16, (int)n_src, (int)n_beams, 6, kpad, n_beams, bk, bn / 2))
-            return LYEM_ERR_CUDA;
-        if (bk == 64)
-            e = bf16 ? launch_tc<64, 256, true, true>(ma, mb_half, p, stream, &done)
-                     : launch_tc<64, 256, false, true>(ma, mb_half, p, stream, &done);
-        else
-            e = bf16 ? launch_tc<32, 256, true, true>(ma, mb_half, p, stream, &done)
-                     : launch_tc<32, 256, false, true>(ma, mb_half, p, stream, &done);
-    }
-    if (e == cudaSuccess && !done)
-        e = bn == 256 ? launch_single<256>(bk, bf16, ma, mb, p, stream)
-            : bn == 128 ? launch_single<128>(bk, bf16, ma, mb, p, stream)
-                        : launch_single<64>(bk, bf16, ma, mb, p, stream);
+    const cudaError_t e = bn == 256   ? launch_bn<256>(bk, bf16, ma, mb, p, stream)
+                          : bn == 128 ? launch_bn<128>(bk, bf16, ma, mb, p, stream)
+                                      : launch_bn<64>(bk, bf16, ma, mb, p, stream);
     if (e != cudaSuccess) {
         record_cuda_error(e);
         return LYEM_ERR_CUDA;

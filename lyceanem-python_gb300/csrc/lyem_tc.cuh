@@ -67,27 +67,6 @@ __device__ __forceinline__ void commit(uint32_t mbar) {
                  : "memory");
 }
 
-// As commit, arriving on the mbarrier at the same shared-memory offset in every CTA of the cluster named by
-// cta_mask (bit i = CTA rank i).
-__device__ __forceinline__ void commit_mc(uint32_t mbar, uint16_t cta_mask) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-                     mbar),
-                 "h"(cta_mask)
-                 : "memory");
-}
-
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-
-// Barrier of every thread of every CTA of the cluster, ordering the shared-memory writes before it (mbarrier
-// initialisation included) before the other CTAs' accesses after it.
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -170,17 +149,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const void* tmap,
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
         "[%5];" ::"r"(dst_smem),
         "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(mbar)
-        : "memory");
-}
-
-// As tma_load_3d, writing the box to the same shared-memory offset in every CTA of the cluster named by
-// cta_mask and completing bytes on the mbarrier at the same offset in each of them.
-__device__ __forceinline__ void tma_load_3d_mc(uint32_t dst_smem, const void* tmap, int x, int y, int z, uint32_t mbar,
-                                               uint16_t cta_mask) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, "
-        "{%2, %3, %4}], [%5], %6;" ::"r"(dst_smem),
-        "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(mbar), "h"(cta_mask)
         : "memory");
 }
 

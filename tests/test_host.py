@@ -154,3 +154,16 @@ def test_time_map_source_chunks_vs_oracle(limit_div, spread):
     otm, owake = O.time_map(amp, arrival, pair, n_src, n_snk, exc, fs, S, map_bytes_limit=limit)
     assert wake == owake
     assert np.abs(tm.numpy() - otm).max() <= 1e-12 * np.abs(otm).max()
+
+
+def test_no_cluster_multicast_in_the_kernels():
+    """Any rank of a multi-GPU job loads the library, so no kernel of it may hold a copy or a commit that writes to
+    several CTAs of a cluster."""
+    import glob
+    import os
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    files = glob.glob(os.path.join(root, "lyceanem-python_gb300", "csrc", "*.cu*"))
+    assert files
+    for path in files:
+        with open(path) as f:
+            assert "multicast::" not in f.read(), path

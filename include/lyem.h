@@ -158,7 +158,9 @@ LYEM_API int lyem_spatial_order(const float *d_points, int64_t n_points, int32_t
  * Optional outputs (NULL to skip): d_pair_out [n_src, n_snk, 6] (the
  * reference's scattering network layout, zero for blocked pairs), d_mask_bits
  * [n_src, ceil(n_snk/32)] uint32 (bit m%32 of word m/32 = visible),
- * d_counters uint64[2] incremented by (visible pairs, ray/triangle tests),
+ * d_counters uint64[2] incremented by (visible pairs, ray/triangle tests:
+ * brute force counts those that decide a ray's outcome, up to its first hit in
+ * triangle order, though a warp drops most triangles for all its rays at once),
  * d_src_visible int32[n_src] / d_snk_visible int32[n_snk] incremented by the
  * visible pairs of each source / sink.
  * d_src_order / d_snk_order (NULL = index order): permutations from

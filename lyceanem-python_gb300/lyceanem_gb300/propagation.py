@@ -158,7 +158,8 @@ def pair_stage(src_pos, src_E, snk_pos, snk_nrm, *, beta, alpha=0.0, tris=None, 
         sink[m, c] (+)= sum_n W[n, c] * S[n, m, c]
     (W = src_W or 1), .pairs the per-pair network complex64 [n_src,n_snk,3]
     when want_pairs, and .mask_bits the visibility bit mask when want_mask.
-    counters (int64 [2]) accumulates (visible pairs, ray/triangle tests);
+    counters (int64 [2]) accumulates (visible pairs, ray/triangle tests; by brute force the tests decided, see
+    include/lyem.h);
     src_visible / snk_visible (int32 [n_src] / [n_snk]) accumulate visible pairs
     per source / per sink.
     src_order / snk_order (int32, e.g. from spatial_order) set the processing

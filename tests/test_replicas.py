@@ -59,3 +59,14 @@ def test_reference_arm_other_ranks_exit_quietly():
     r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1",
                         "--warmup", "0"], env=env, capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == ""
+
+
+def test_brute_force_roofline_claims_no_executed_tests():
+    """The brute-force counter holds decided tests, of which most are not made: no achieved rate comes from it (64
+    elements, 2,664 sinks, 1,024 triangles in 87 us would be 1.6 times the FMA peak)."""
+    import bench
+    args = ("brute_stage_kernel", 1.75e8, 1.75e8, 0.087, 0.1, 38.3, None)
+    r = bench.stage_roofline(*args, executed=False)
+    assert r["frac"] is None and r["achieved"] is None and r["effective_frac"] > 1
+    g = bench.stage_roofline("grid_stage_kernel", 1e9, 1e12, 1.0, 1.2, 38.3, None, executed=True)
+    assert abs(g["achieved"] - 30.0) < 1e-9 and abs(g["frac"] - 30.0 / 38.3) < 1e-9

@@ -204,3 +204,12 @@ class Brute_Force_acceleration_structure:
 
     def sink_field(self, source_mesh, sink_mesh, alpha, beta, wavelength=None, self_to_self=False):
         return self.device.sink_field(source_mesh, sink_mesh, alpha, beta, self_to_self)
+
+
+def own_networks(acc):
+    """Whether acc's networks are those of this module's structures: a subclass or an instance with a
+    calculate_scattering of its own, or with another kind of device scene, is asked for each network."""
+    return (getattr(type(acc), "calculate_scattering", None) in
+            (Tile_acceleration_structure.calculate_scattering, Brute_Force_acceleration_structure.calculate_scattering)
+            and "calculate_scattering" not in getattr(acc, "__dict__", {})
+            and type(getattr(acc, "device", None)) is _DeviceScene)

@@ -96,7 +96,7 @@ def calculate_scattering_cuda(alpha, beta, wavelength, acceleration_structure, s
     """Per-element network total = S0 (+ S1 @ S2 per component), complex64 [N, M, 3]
     (lyceanem/models/frequency_domain.py:195-264)."""
     acc = acceleration_structure
-    if scatter_depth > 0 and isinstance(getattr(acc, "device", None), acceleration_structures._DeviceScene):
+    if scatter_depth > 0 and acceleration_structures.own_networks(acc):
         return _bounce_network(acc.device, acceleration_structures.em_float(alpha),
                                acceleration_structures.em_float(beta), scatter_depth, source_mesh, sink_mesh, scatter_mesh,
                                chunks)

@@ -840,6 +840,48 @@ def test_masks_bit_exact_to_reference_device_code(case):
         assert np.abs(got - ref_f).max() / np.abs(ref_f).max() < 1e-3
 
 
+def _element_scene(seed, N, Pn, M):
+    from lyceanem_gb300.geometry import Mesh
+    src, snk, snk_n, v, f, E = random_scene(seed, n_src=N, n_snk=M, n_tris=60)
+    rng = np.random.default_rng(seed)
+    scat = rng.uniform(-1, 1, (Pn, 3)).astype(np.float32)
+    scat_n = rng.normal(size=(Pn, 3))
+    scat_n = (scat_n / np.linalg.norm(scat_n, axis=1, keepdims=True)).astype(np.float32)
+    ap = Mesh(src, point_data={"Normals": np.tile([[0, 0, 1.0]], (N, 1)), "ex": E[:, 0], "ey": E[:, 1], "ez": E[:, 2]})
+    return ap, Mesh(snk, point_data={"Normals": snk_n}), Mesh(scat, point_data={"Normals": scat_n}), Mesh(v, [("triangle", f)])
+
+
+@pytest.mark.parametrize("depth,calls", [(0, 1), (1, 3), (2, 3)])
+def test_structure_with_its_own_networks_is_asked_for_them(depth, calls):
+    """calculate_scattering of a subclass, or set on an instance, gives every network of the per-element composition."""
+    from lyceanem_gb300.models import acceleration_structures as A
+    from lyceanem_gb300.models import frequency_domain as FD
+    ap, sk, sc, solid = _element_scene(5, 6, 20, 40)
+
+    class Twice(A.Brute_Force_acceleration_structure):
+        seen = 0
+
+        def calculate_scattering(self, *a, **k):
+            self.seen += 1
+            return np.float32(2) * super().calculate_scattering(*a, **k)
+
+    acc = Twice(solid)
+    got = FD.calculate_scattering_cuda(0.0, 30.0, 0.2, acc, depth, ap, sk, sc)
+    assert acc.seen == calls
+    # 2 S0 + (2 S1) (2 S2(2 e_p)), S2 linear in its excitation: 2 S0 + 8 S1 S2
+    plain = A.Brute_Force_acceleration_structure(solid)
+    S0 = FD.calculate_scattering_cuda(0.0, 30.0, 0.2, plain, 0, ap, sk, sc)
+    one = FD.calculate_scattering_cuda(0.0, 30.0, 0.2, plain, 1, ap, sk, sc)
+    want = 2 * S0 if depth != 1 else 2 * S0 + 8 * (one - S0)
+    assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
+    acc = A.Tile_acceleration_structure(solid, 4)
+    seen = []
+    orig = acc.calculate_scattering
+    acc.calculate_scattering = lambda *a, **k: (seen.append(1), orig(*a, **k))[1]
+    FD.calculate_scattering_cuda(0.0, 30.0, 0.2, acc, depth, ap, sk, sc)
+    assert len(seen) == calls
+
+
 def test_scene_cache_reuses_device_grid():
     """Repeated model calls on the same solid reuse its device triangles and grid; the results are
     identical and a different solid builds a new scene."""

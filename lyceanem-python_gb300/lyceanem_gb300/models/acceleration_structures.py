@@ -88,32 +88,33 @@ class _DeviceScene:
         return P.pair_stage(src, E, snk, snk_n, beta=beta, alpha=alpha, tris=self.tris, grid=self.grid,
                             self_to_self=self_to_self, **kw)
 
-    def _chunk_networks(self, src, E, snk, snk_n, alpha, beta, self_to_self, chunk_count):
+    def chunk_networks(self, src, E, snk, snk_n, alpha, beta, self_to_self, chunk_count, out=None):
+        """(a, b, network of sources a .. b - 1) over the source chunks of the reference's loop, so that the untested
+        pair of equal indices is the same one; each network in out's rows a .. b - 1 if out is given."""
         for a, b in _chunks(src.shape[0], chunk_count):
-            yield self.stage(src[a:b], E[a:b], snk, snk_n, alpha, beta, self_to_self, want_pairs=True,
-                             traversal=P.source_schedule(src[a:b], self.grid)).pairs
+            yield a, b, self.stage(src[a:b], E[a:b], snk, snk_n, alpha, beta, self_to_self, want_pairs=True,
+                                   pairs_out=None if out is None else out[a:b],
+                                   traversal=P.source_schedule(src[a:b], self.grid)).pairs
 
     def network_tensor(self, src, E, snk, snk_n, alpha, beta, self_to_self, chunk_count):
-        """The network complex64 [N, M, 3] as a CUDA tensor; sources (numpy) and their excitations E in the chunks of
-        the reference's loop, so that the untested pair of equal indices is the same one."""
-        parts = list(self._chunk_networks(src, E, snk, snk_n, alpha, beta, self_to_self, chunk_count))
-        if not parts:
-            return torch.zeros((0, snk.shape[0], 3), dtype=torch.complex64, device=snk.device)
-        return parts[0] if len(parts) == 1 else torch.cat(parts)
+        """The network complex64 [N, M, 3] as a CUDA tensor (sources and excitations E numpy or CUDA)."""
+        out = torch.empty((src.shape[0], snk.shape[0], 3), dtype=torch.complex64, device=snk.device)
+        for _ in self.chunk_networks(src, E, snk, snk_n, alpha, beta, self_to_self, chunk_count, out):
+            pass
+        return out
 
     def network(self, source_mesh, sink_mesh, alpha, beta, self_to_self, chunk_count):
         src = np.asarray(source_mesh.points, dtype=np.float32)
         snk, snk_n = sink_tensors(sink_mesh)
         E = _cvec_from_point_data(source_mesh)
         out = None
-        at = 0
-        for part in self._chunk_networks(src, E, snk, snk_n, alpha, beta, self_to_self, chunk_count):
-            if part.shape[0] == src.shape[0]:
+        for a, b, part in self.chunk_networks(src, E, snk, snk_n, alpha, beta, self_to_self, chunk_count):
+            if b - a == src.shape[0]:
                 return part.cpu().numpy()
             if out is None:
                 out = np.empty((src.shape[0], snk.shape[0], 3), dtype=np.complex64)
-            out[at:at + part.shape[0]] = part.cpu().numpy()
-            at += part.shape[0]
+            out[a:b] = part.cpu().numpy()
+            del part  # before the next chunk's is allocated
         return np.zeros((src.shape[0], snk.shape[0], 3), dtype=np.complex64) if out is None else out
 
     def sink_field(self, source_mesh, sink_mesh, alpha, beta, self_to_self=False):

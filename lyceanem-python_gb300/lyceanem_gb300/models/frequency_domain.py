@@ -96,10 +96,9 @@ def calculate_scattering_cuda(alpha, beta, wavelength, acceleration_structure, s
     """Per-element network total = S0 (+ S1 @ S2 per component), complex64 [N, M, 3]
     (lyceanem/models/frequency_domain.py:195-264)."""
     acc = acceleration_structure
-    if scatter_depth > 0 and acceleration_structures.own_networks(acc):
+    if scatter_depth == 1 and acceleration_structures.own_networks(acc):
         return _bounce_network(acc.device, acceleration_structures.em_float(alpha),
-                               acceleration_structures.em_float(beta), scatter_depth, source_mesh, sink_mesh, scatter_mesh,
-                               chunks)
+                               acceleration_structures.em_float(beta), source_mesh, sink_mesh, scatter_mesh, chunks)
     total = acc.calculate_scattering(source_mesh, sink_mesh, alpha, beta, wavelength, chunk_count=chunks,
                                      self_to_self=False)
     if scatter_depth == 0:
@@ -121,9 +120,10 @@ def calculate_scattering_cuda(alpha, beta, wavelength, acceleration_structure, s
     return total
 
 
-def _bounce_network(dev, alpha, beta, scatter_depth, source_mesh, sink_mesh, scatter_mesh, chunks):
+def _bounce_network(dev, alpha, beta, source_mesh, sink_mesh, scatter_mesh, chunks):
     """calculate_scattering_cuda with one bounce on this package's structures: the networks of its three stages stay on
-    the device (as host arrays they went down and up again: 64 elements, 800 scatter points, 2,701 sinks 9.4 -> 1.4 ms)."""
+    the device (as host arrays they went down and up again: 64 elements, 800 scatter points, 2,701 sinks 9.4 -> 1.4 ms).
+    `chunks` bounds what they take: of the scatter -> sink network, the largest, one chunk is there at a time."""
     src = np.asarray(source_mesh.points, dtype=np.float32)
     scat = np.asarray(scatter_mesh.points, dtype=np.float32)
     E = acceleration_structures._cvec_from_point_data(source_mesh)
@@ -135,10 +135,10 @@ def _bounce_network(dev, alpha, beta, scatter_depth, source_mesh, sink_mesh, sca
     host = e_p.cpu().numpy()
     for c, k in enumerate(("ex", "ey", "ez")):
         scatter_mesh.point_data[k] = host[:, c].copy()
-    if scatter_depth == 1:
-        S2 = dev.network_tensor(scat, e_p, snk, snk_n, alpha, beta, False, chunks)
+    for a, b, S2 in dev.chunk_networks(scat, e_p, snk, snk_n, alpha, beta, False, chunks):
         for c in range(3):
-            total[:, :, c] += S1[:, :, c] @ S2[:, :, c]
+            total[:, :, c] += S1[:, a:b, c] @ S2[:, :, c]
+        del S2  # before the next chunk's is allocated
     return total.cpu().numpy()
 
 

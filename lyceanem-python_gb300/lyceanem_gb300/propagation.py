@@ -151,13 +151,14 @@ def _check_buffer(name, t, dtype, n, exact):
 def pair_stage(src_pos, src_E, snk_pos, snk_nrm, *, beta, alpha=0.0, tris=None, grid=None, src_W=None,
                self_to_self=False, cull=True, eps=EPSILON, sink_out=None, accumulate=False, want_pairs=False,
                want_mask=False, counters=None, src_visible=None, snk_visible=None, src_order=None, snk_order=None,
-               src_chunk=0, traversal=0, workspace=None):
+               src_chunk=0, traversal=0, workspace=None, pairs_out=None):
     """Visibility + fused field of every (source, sink) pair.
 
     Returns a StageResult whose .sink is complex64 [n_snk,3] with
         sink[m, c] (+)= sum_n W[n, c] * S[n, m, c]
     (W = src_W or 1), .pairs the per-pair network complex64 [n_src,n_snk,3]
-    when want_pairs, and .mask_bits the visibility bit mask when want_mask.
+    when want_pairs (written to pairs_out, a contiguous tensor of that shape,
+    if given), and .mask_bits the visibility bit mask when want_mask.
     counters (int64 [2]) accumulates (visible pairs, ray/triangle tests; by brute force the tests decided, see
     include/lyem.h);
     src_visible / snk_visible (int32 [n_src] / [n_snk]) accumulate visible pairs
@@ -210,7 +211,14 @@ def pair_stage(src_pos, src_E, snk_pos, snk_nrm, *, beta, alpha=0.0, tris=None, 
         sink_out = torch.empty((M, 3), dtype=torch.complex64, device=dev)
         accumulate = False
     alloc = torch.empty if N == rows else torch.zeros  # rows left out of a subset stay zero
-    pairs = alloc((rows, M, 3), dtype=torch.complex64, device=dev) if want_pairs else None
+    pairs = None
+    if pairs_out is not None:
+        if not (isinstance(pairs_out, torch.Tensor) and pairs_out.device == dev and pairs_out.dtype == torch.complex64
+                and tuple(pairs_out.shape) == (rows, M, 3) and pairs_out.is_contiguous()):
+            raise ValueError(f"pairs_out must be a contiguous complex64 CUDA tensor of shape {(rows, M, 3)}")
+        pairs = pairs_out if N == rows else pairs_out.zero_()
+    elif want_pairs:
+        pairs = alloc((rows, M, 3), dtype=torch.complex64, device=dev)
     words = (M + 31) // 32
     mbits = alloc((rows, words), dtype=torch.int32, device=dev) if want_mask else None
     # the transposed schedule (traversal 38) takes 32 sources per block, whatever src_chunk says

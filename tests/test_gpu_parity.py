@@ -882,6 +882,39 @@ def test_structure_with_its_own_networks_is_asked_for_them(depth, calls):
     assert len(seen) == calls
 
 
+@pytest.mark.parametrize("chunks", [2, 5])
+def test_chunks_bound_the_device_memory_of_element_networks(chunks):
+    """Per-element networks of N x P, N x M and P x M pairs: with chunks, one chunk of the largest is on the device at a
+    time beside the two others and one product's operands and result (a third of their networks each); above one bounce,
+    where no product is formed, one chunk of one network."""
+    from lyceanem_gb300.models import acceleration_structures as A
+    from lyceanem_gb300.models import frequency_domain as FD
+    N, Pn, M = 16, 600, 3000
+    ap, sk, sc, solid = _element_scene(7, N, Pn, M)
+    acc = A.Tile_acceleration_structure(solid, 4)
+    nets = {k: 24 * a * b for k, a, b in (("S0", N, M), ("S1", N, Pn), ("S2", Pn, M))}
+
+    def peak(depth, chunks):
+        FD.calculate_scattering_cuda(0.0, 30.0, 0.2, acc, depth, ap, sk, sc, chunks)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        out = FD.calculate_scattering_cuda(0.0, 30.0, 0.2, acc, depth, ap, sk, sc, chunks)
+        return torch.cuda.max_memory_allocated() - before, out
+
+    one, whole = peak(1, 1)
+    some, parts = peak(1, chunks)
+    step = nets["S2"] / chunks
+    stage_ws = 24 * M * (-(-Pn // chunks))  # a stage's partial sums, one row of sinks a source at most
+    rest = (nets["S0"] + nets["S1"]) * 4 / 3 + 2 * stage_ws + (8 << 20)
+    assert some <= step * 4 / 3 + rest
+    assert one >= nets["S2"]  # (the measure sees the networks)
+    # the same composition, the untested pairs of equal indices apart (they are those of each chunk)
+    assert parts.shape == whole.shape and np.isfinite(parts).all()
+    deep, _ = peak(2, chunks)
+    assert deep <= step + 2 * stage_ws + (8 << 20)
+
+
 def test_scene_cache_reuses_device_grid():
     """Repeated model calls on the same solid reuse its device triangles and grid; the results are
     identical and a different solid builds a new scene."""

@@ -98,6 +98,8 @@ class _DeviceScene:
 
     def network_tensor(self, src, E, snk, snk_n, alpha, beta, self_to_self, chunk_count):
         """The network complex64 [N, M, 3] as a CUDA tensor (sources and excitations E numpy or CUDA)."""
+        if chunk_count == 1 and src.shape[0]:
+            return next(self.chunk_networks(src, E, snk, snk_n, alpha, beta, self_to_self, 1))[2]
         out = torch.empty((src.shape[0], snk.shape[0], 3), dtype=torch.complex64, device=snk.device)
         for _ in self.chunk_networks(src, E, snk, snk_n, alpha, beta, self_to_self, chunk_count, out):
             pass

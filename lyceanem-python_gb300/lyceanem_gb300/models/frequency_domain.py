@@ -136,8 +136,9 @@ def _bounce_network(dev, alpha, beta, source_mesh, sink_mesh, scatter_mesh, chun
     for c, k in enumerate(("ex", "ey", "ez")):
         scatter_mesh.point_data[k] = host[:, c].copy()
     for a, b, S2 in dev.chunk_networks(scat, e_p, snk, snk_n, alpha, beta, False, chunks):
+        part = S1[:, a:b]
         for c in range(3):
-            total[:, :, c] += S1[:, a:b, c] @ S2[:, :, c]
+            total[:, :, c] += part[:, :, c] @ S2[:, :, c]
         del S2  # before the next chunk's is allocated
     return total.cpu().numpy()
 

@@ -364,8 +364,13 @@ LYEM_API int lyem_pair_stage(const float* d_src_pos, const float* d_src_E, const
     int chunk = src_chunk > 0 ? src_chunk : auto_src_chunk(n_src, n_snk, use_grid);
     chunk = std::min(chunk, use_grid ? grid_max_src_chunk() : brute_max_src_chunk());
     if (use_grid && traversal == 38) chunk = transposed_src_chunk();  // one lane per source of a chunk
+    // 39: the lockstep and the transposed schedule are both launched, and the one that the sources' extent, found on the
+    // device, does not choose ends at once (its blocks cost 1 % of the other's at most).  The choice lies behind the
+    // partial sums, in the workspace's last 256 bytes.
+    const bool choose = use_grid && traversal == 39;
     if ((n_snk + stage_block_threads() - 1) / stage_block_threads() > 0x7fffffffLL) return LYEM_ERR_OVERFLOW;
-    const size_t need = stage_ws_bytes(n_src, n_snk, chunk);
+    size_t need = stage_ws_bytes(n_src, n_snk, chunk);
+    if (choose) need = std::max(need, stage_ws_bytes(n_src, n_snk, transposed_src_chunk()));
     if (!d_ws || ws_bytes < need) return LYEM_ERR_WORKSPACE;
 
     StageParams p;
@@ -407,17 +412,17 @@ LYEM_API int lyem_pair_stage(const float* d_src_pos, const float* d_src_E, const
     p.src_order = d_src_order;
     p.snk_order = d_snk_order;
     const bool two_phase = (traversal >= 101 && traversal <= 164) || (traversal >= 201 && traversal <= 264);
-    if ((traversal < 0 || traversal > 38 || traversal == 37) && !two_phase) return LYEM_ERR_INVALID;
+    if ((traversal < 0 || traversal > 39 || traversal == 37) && !two_phase) return LYEM_ERR_INVALID;
     static const int kCapped[3] = {-10, -12, -16};  // traversal 34, 35, 36
     if (two_phase) {
         p.refill_lanes = traversal < 200 ? -116 : -112;
         p.near_dist = (float)(traversal % 100) * (use_grid ? grid_cell : 1.f);
     } else {
-        p.refill_lanes = traversal == 0 ? -16 : traversal == 1 ? 0 : traversal <= 33 ? traversal - 1
+        p.refill_lanes = traversal == 0 || traversal == 39 ? -16 : traversal == 1 ? 0 : traversal <= 33 ? traversal - 1
                          : traversal == 38 ? -38 : kCapped[traversal - 34];
     }
     // permuted sinks, and the transposed schedule's warps, set their mask bits one by one
-    if (d_mask_bits && (d_snk_order || (use_grid && traversal == 38))) {
+    if (d_mask_bits && (d_snk_order || (use_grid && traversal >= 38 && !two_phase))) {
         if (d_src_order) {  // (it may list any rows)
             zero_mask_rows_kernel<<<blocks_for(n_src * p.mask_words, 256), 256, 0, s>>>(d_mask_bits, d_src_order, n_src,
                                                                                        p.mask_words);
@@ -427,11 +432,22 @@ LYEM_API int lyem_pair_stage(const float* d_src_pos, const float* d_src_E, const
             LYEM_CK(cudaMemsetAsync(d_mask_bits, 0, sizeof(uint32_t) * (size_t)n_src * (size_t)p.mask_words, s));
         }
     }
-    LYEM_CK(launch_pair_stage(p, cull, s));
-    if (d_sink_out) {
-        const long long chunks = (n_src + chunk - 1) / chunk;
-        LYEM_CK(launch_reduce_partials(p.partial, chunks, n_snk, d_sink_out, accumulate, s));
+    const long long chunks = (n_src + chunk - 1) / chunk;
+    long long t_chunks = 0;
+    int* choice = nullptr;
+    if (choose) {
+        choice = reinterpret_cast<int*>(static_cast<char*>(d_ws) + (need - 256));
+        LYEM_CK(launch_source_choice(d_src_pos, d_src_order, n_src, grid_cell, choice, s));
+        p.choice = choice;
+        StageParams t = p;
+        t.choice_is = 1;
+        t.refill_lanes = -38;
+        t.src_chunk = transposed_src_chunk();
+        t_chunks = (n_src + t.src_chunk - 1) / t.src_chunk;
+        LYEM_CK(launch_pair_stage(t, cull, s));
     }
+    LYEM_CK(launch_pair_stage(p, cull, s));
+    if (d_sink_out) LYEM_CK(launch_reduce_partials(p.partial, chunks, n_snk, d_sink_out, accumulate, s, choice, t_chunks));
     return LYEM_OK;
 }
 

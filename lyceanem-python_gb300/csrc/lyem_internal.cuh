@@ -57,6 +57,8 @@ struct StageParams {
                        // -10 / -12 / -16 = lockstep with registers capped for that many blocks per SM,
                        // -116 / -112 = two phases split at near_dist, capped for 16 / 12 blocks per SM
     int snk_per_warp;  // transposed schedule: sinks a warp takes (set at launch)
+    const int* choice; // if given, the launch's blocks do their work only where *choice == choice_is
+    int choice_is;
     float near_dist;   // two-phase schedule: ray parameter (m) where phase 1 hands open rays to phase 2
     // outputs
     float* partial;              // [n_chunks, n_snk, 6]
@@ -87,8 +89,14 @@ cudaError_t fma_probe(long long iters, double* fma_per_s, cudaStream_t stream);
 
 // Host-side launchers (lyem_stage.cu).
 cudaError_t launch_pair_stage(const StageParams& p, int cull, cudaStream_t stream);
+// choice: if given and *choice != 0, the partial sums are those of chosen_chunks chunks instead.
 cudaError_t launch_reduce_partials(const float* partial, long long n_chunks, long long n_snk, float* out,
-                                   int accumulate, cudaStream_t stream);
+                                   int accumulate, cudaStream_t stream, const int* choice = nullptr,
+                                   long long chosen_chunks = 0);
+// *choice = 1 where the sources lie within kCompactCells grid cells of each other, else 0.
+cudaError_t launch_source_choice(const float* src_pos, const int* src_order, long long n_src, float cell, int* choice,
+                                 cudaStream_t stream);
+constexpr double kCompactCells = 4.0;  // (propagation.source_schedule: host arrays)
 int stage_block_threads();
 // Sources per thread block of a pair stage when the caller passes 0 (lyem_capi.cu).
 int auto_src_chunk(long long n_src, long long n_snk, bool grid);

@@ -494,6 +494,7 @@ constexpr int kTwoPhase12 = 6;
 // scene 448 -> 440 ms).
 template <bool CULL, bool WEIGHTED, bool PAIR_OUT, bool MASK_OUT, int MODE, bool COUNT = true>
 __global__ void __launch_bounds__(kThreads, MODE == kLockstep10 ? 10 : (MODE == kLockstep12 || MODE == kTwoPhase12) ? 12 : (MODE == kLockstep16 || MODE == kTwoPhase16) ? 16 : 1) grid_stage_kernel(const StageParams p) {
+    if (p.choice && *p.choice != p.choice_is) return;
     // 32-bit indices (fewer live registers in the walk): the entry point keeps
     // n_src and n_snk below 2^31 - 256
     const int tid = threadIdx.x;
@@ -715,6 +716,7 @@ static int transposed_sinks(long long n_src, long long n_snk) {
 
 template <bool CULL, bool WEIGHTED, bool PAIR_OUT, bool MASK_OUT, bool COUNT>
 __global__ void __launch_bounds__(kThreads, 16) grid_transposed_kernel(const StageParams p) {
+    if (p.choice && *p.choice != p.choice_is) return;
     const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long chunk = p.chunk_base + (long long)blockIdx.y;
@@ -798,7 +800,9 @@ __global__ void __launch_bounds__(kThreads, 16) grid_transposed_kernel(const Sta
 // One thread per element left the loads of its chunks one behind the other: 15,984 elements of 64 chunks 16.7 -> 8.3 us.
 constexpr int kReduceParts = 8;
 __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, long long n_chunks,
-                                                             long long n_elem, float* __restrict__ out, int accumulate) {
+                                                             long long n_elem, float* __restrict__ out, int accumulate,
+                                                             const int* __restrict__ choice, long long chosen_chunks) {
+    if (choice && *choice) n_chunks = chosen_chunks;
     __shared__ double s_part[kReduceParts][32];
     const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
     const long long per = (n_chunks + kReduceParts - 1) / kReduceParts;
@@ -820,6 +824,56 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
         }
         __syncthreads();
     }
+}
+
+// Extent of the sources, by one block: 16,384 of them are 200 KB, and the stage that waits for it takes milliseconds.
+__global__ void __launch_bounds__(1024) source_choice_kernel(const float* __restrict__ pos, const int* __restrict__ order,
+                                                            int n, float cell, int* __restrict__ choice) {
+    __shared__ float s_lo[3][32], s_hi[3][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    bool bad = false;
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        const float* p = pos + 3 * (long long)(order ? order[i] : i);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float v = p[k];
+            bad |= !(fabsf(v) < INFINITY);
+            lo[k] = fminf(lo[k], v);
+            hi[k] = fmaxf(hi[k], v);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+            hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+        }
+        if (lane == 0) {
+            s_lo[k][warp] = lo[k];
+            s_hi[k][warp] = hi[k];
+        }
+    }
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x == 0) {
+        double d2 = 0.0;
+        for (int k = 0; k < 3; ++k) {
+            float a = s_lo[k][0], b = s_hi[k][0];
+            for (int w = 1; w < 32; ++w) {
+                a = fminf(a, s_lo[k][w]);
+                b = fmaxf(b, s_hi[k][w]);
+            }
+            const double e = (double)(b - a);
+            d2 += e * e;
+        }
+        *choice = !bad && sqrt(d2) <= kCompactCells * (double)cell;
+    }
+}
+
+cudaError_t launch_source_choice(const float* src_pos, const int* src_order, long long n_src, float cell, int* choice,
+                                 cudaStream_t stream) {
+    source_choice_kernel<<<1, 1024, 0, stream>>>(src_pos, src_order, (int)n_src, cell, choice); note_launches(1);
+    return cudaGetLastError();
 }
 
 template <bool CULL, bool WEIGHTED, bool PAIR_OUT, bool MASK_OUT>
@@ -893,11 +947,13 @@ cudaError_t launch_pair_stage(const StageParams& p, int cull, cudaStream_t strea
 }
 
 cudaError_t launch_reduce_partials(const float* partial, long long n_chunks, long long n_snk, float* out,
-                                   int accumulate, cudaStream_t stream) {
+                                   int accumulate, cudaStream_t stream, const int* choice,
+                                   long long chosen_chunks) {
     const long long n_elem = 6 * n_snk;
     if (n_elem == 0) return cudaSuccess;
     const unsigned blocks = capped_blocks(n_elem, 32, 64);
-    reduce_partials_kernel<<<blocks, 256, 0, stream>>>(partial, n_chunks, n_elem, out, accumulate); note_launches(1);
+    reduce_partials_kernel<<<blocks, 256, 0, stream>>>(partial, n_chunks, n_elem, out, accumulate, choice, chosen_chunks);
+    note_launches(1);
     return cudaGetLastError();
 }
 

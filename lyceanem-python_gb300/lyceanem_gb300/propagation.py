@@ -221,9 +221,11 @@ def pair_stage(src_pos, src_E, snk_pos, snk_nrm, *, beta, alpha=0.0, tris=None, 
         pairs = alloc((rows, M, 3), dtype=torch.complex64, device=dev)
     words = (M + 31) // 32
     mbits = alloc((rows, words), dtype=torch.int32, device=dev) if want_mask else None
-    # the transposed schedule (traversal 38) takes 32 sources per block, whatever src_chunk says
-    wchunk = 32 if (grid is not None and traversal == 38) else int(src_chunk)
-    need = lib.lyem_pair_stage_workspace(N, M, T, int(grid is not None), wchunk)
+    # the transposed schedule (traversal 38, and 39 where it is chosen) takes 32 sources per block, whatever src_chunk says
+    need = 0 if grid is not None and traversal == 38 else \
+        lib.lyem_pair_stage_workspace(N, M, T, int(grid is not None), int(src_chunk))
+    if grid is not None and traversal in (38, 39):
+        need = max(need, lib.lyem_pair_stage_workspace(N, M, T, 1, 32))
     if workspace is None or workspace.numel() < need:
         workspace = _ws(need, dev)
     st = lib.lyem_pair_stage(_p(sp), _p(torch.view_as_real(E)), _p(None if W is None else torch.view_as_real(W)), N,
@@ -255,27 +257,21 @@ def source_schedule(src, grid, n_snk=None):
     elements of an array), so that a warp's rays to a sink cross the same cells; otherwise the default (0).
     Elements spread over 4.2 cells: 1.14 -> 0.88 ms to 16,471 sinks, 0.58 -> 0.38 ms to 5,000 scatter points (256
     elements, 40,000 triangles); over 8.5 cells the gain to 65,341 sinks is gone (3.33 against 3.61 ms).
-    A device tensor is reduced on the device (one small synchronisation); given n_snk, the sinks of the stage, that
-    is done for stages of at least 2^20 pairs only (about 0.3 ms), and with few sinks (scatter_schedule) not at all.
-    Under stream capture, which a synchronisation would break, the default is kept."""
+    Host arrays are looked at here.  For CUDA tensors the choice is left to the device (traversal 39: no
+    synchronisation, and none under capture), except that a stage whose sinks, n_snk if given, are few
+    (scatter_schedule) takes the transposed schedule wherever its sources lie (256 / 1,024 sources all over a scene of
+    20,000 triangles to 1,000 / 2,000 sinks: 0.316 -> 0.289 / 1.009 -> 0.977 ms)."""
     if grid is None:
         return 0
     if isinstance(src, torch.Tensor) and src.is_cuda:
-        a = src.reshape(-1, 3)
-        if a.shape[0] == 0:
+        if src.numel() == 0:
             return 0
-        if n_snk is not None and scatter_schedule(n_snk, grid):
-            return 38
-        if (n_snk is not None and a.shape[0] * n_snk < 1 << 20) or torch.cuda.is_current_stream_capturing():
-            return 0
-        lo, hi = torch.aminmax(a.float(), dim=0)
-        ext = (hi - lo).double().cpu().numpy()
-    else:
-        import numpy as np
-        a = np.asarray(src, np.float64).reshape(-1, 3)
-        if a.shape[0] == 0:
-            return 0
-        ext = a.max(0) - a.min(0)
+        return 38 if n_snk is not None and scatter_schedule(n_snk, grid) else 39
+    import numpy as np
+    a = np.asarray(src, np.float64).reshape(-1, 3)
+    if a.shape[0] == 0:
+        return 0
+    ext = a.max(0) - a.min(0)
     return 38 if float((ext ** 2).sum()) ** 0.5 <= 4.0 * grid.cell else 0
 
 

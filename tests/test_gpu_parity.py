@@ -915,6 +915,75 @@ def test_chunks_bound_the_device_memory_of_element_networks(chunks):
     assert deep <= step + 2 * stage_ws + (8 << 20)
 
 
+@pytest.mark.parametrize("n_src,n_snk", [(1, 1), (31, 3), (33, 130), (300, 700), (2080, 5000)])
+@pytest.mark.parametrize("spread", ["point", "below", "above", "wide", "nan"])
+def test_schedule_chosen_on_the_device(n_src, n_snk, spread):
+    """Traversal 39: the transposed schedule where the sources' extent is at most four cells, else the lockstep one, bit
+    for bit what an explicit choice gives, with every output, orders, a subset and an accumulated sink field."""
+    P = _P()
+    _, snk, snk_n, v, f, E = random_scene(n_src + n_snk, n_src=n_src, n_snk=n_snk, n_tris=200)
+    g = P.UniformGrid(P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f)))
+    rng = np.random.default_rng(n_src)
+    ext = {"point": 0.0, "below": 3.99, "above": 4.01, "wide": 40.0, "nan": 1.0}[spread] * g.cell / 3 ** 0.5
+    u = rng.uniform(0, 1, (n_src, 3))
+    u[0], u[-1] = 0.0, 1.0
+    src = (u * ext + 0.1).astype(np.float32)
+    if spread == "nan":
+        src[n_src // 2, 1] = np.nan
+    compact = spread in ("point", "below") or (n_src == 1 and spread != "nan")
+    same = 38 if compact else 36
+    assert P.source_schedule(src, g) == (38 if compact else 0)
+    src, snk, snk_n, E = (torch.from_numpy(x).cuda() for x in (src, snk, snk_n, E))
+    assert P.source_schedule(src, g) == 39
+    i32 = dict(dtype=torch.int32, device="cuda")
+    o_snk = P.spatial_order(snk)
+    forms = [dict(want_mask=True, want_pairs=True), dict(want_mask=True, snk_order=o_snk), dict(cull=False, eps=1e-7),
+             dict(src_W=E, src_order=torch.arange(n_src - 1, -1, -1, **i32), want_mask=True, snk_order=o_snk)]
+    if n_src > 2:
+        forms.append(dict(src_order=torch.arange(0, n_src - 1, 2, **i32), want_mask=True, want_pairs=True))
+    for kw in forms:
+        res = []
+        for trav in (same, 39):
+            sv, kv, cnt = torch.zeros(n_src, **i32), torch.zeros(n_snk, **i32), torch.zeros(2, dtype=torch.int64, device="cuda")
+            out = torch.full((n_snk, 3), 0.5 + 1j, dtype=torch.complex64, device="cuda")
+            # a subset without the last (or NaN) source may be compact where the whole set is not: choose for it
+            t = trav
+            if trav != 39 and kw.get("src_order") is not None:
+                t = 38 if P.source_schedule(src[kw["src_order"].long()].cpu().numpy(), g) == 38 else 36
+            r = P.pair_stage(src, E, snk, snk_n, beta=30.0, grid=g, traversal=t, src_visible=sv, snk_visible=kv,
+                             counters=cnt, sink_out=out, accumulate=True, **kw)
+            res.append([torch.view_as_real(r.sink), sv, kv, cnt, r.mask_bits, None if r.pairs is None else torch.view_as_real(r.pairs)])
+        for x, y in zip(*res):
+            assert (x is None and y is None) or torch.equal(torch.nan_to_num(x), torch.nan_to_num(y)), kw
+    _no_device_errors()
+
+
+@pytest.mark.parametrize("n_src,n_snk", [(1024, 2000), (300, 4000), (20, 300)])
+def test_device_arrays_enqueue_without_a_wait(n_src, n_snk):
+    """With device arrays, the network and the numba fields only enqueue work: no copy back, no synchronisation."""
+    from lyceanem_gb300 import beam_sweep as BS
+    from lyceanem_gb300.models import frequency_domain as FD
+    P = _P()
+    src, snk, snk_n, v, f, E = random_scene(3, n_src=n_src, n_snk=n_snk, n_tris=100)
+    tris = P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f))
+    st = type("S", (), {"device": type("D", (), {"tris": tris, "grid": P.UniformGrid(tris)})()})()
+    src, snk, snk_n, E = (torch.from_numpy(x).cuda() for x in (src, snk, snk_n, E))
+    scat, scat_n = snk[:50].clone(), snk_n[:50].clone()
+
+    def calls():
+        BS.form_network(src, E, snk, snk_n, beta=30.0, grid=st.device.grid)
+        FD.numba_sink_field(st, src, E, snk, snk_n, 0.0, 30.0, scat, scat_n, scattering=1)
+        FD.numba_per_element(st, src[:20], E[:20], snk, snk_n, 0.0, 30.0)
+    calls()
+    torch.cuda.synchronize()
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        calls()
+    finally:
+        torch.cuda.set_sync_debug_mode("default")
+    _no_device_errors()
+
+
 def test_scene_cache_reuses_device_grid():
     """Repeated model calls on the same solid reuse its device triangles and grid; the results are
     identical and a different solid builds a new scene."""

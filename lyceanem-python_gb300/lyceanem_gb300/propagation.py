@@ -268,6 +268,8 @@ def source_schedule(src, grid, n_snk=None):
             return 0
         return 38 if n_snk is not None and scatter_schedule(n_snk, grid) else 39
     import numpy as np
+    if isinstance(src, torch.Tensor):  # (bfloat16 and tensors with gradients have no numpy form)
+        src = src.detach().double().numpy()
     a = np.asarray(src, np.float64).reshape(-1, 3)
     if a.shape[0] == 0:
         return 0

@@ -167,3 +167,20 @@ def test_no_cluster_multicast_in_the_kernels():
     for path in files:
         with open(path) as f:
             assert "multicast::" not in f.read(), path
+
+
+def test_source_schedule_of_host_forms():
+    """Lists, arrays and host tensors, of a type that numpy does not know and with gradients among them."""
+    import torch
+
+    from lyceanem_gb300 import propagation as P
+    grid = type("G", (), {"cell": 1.0})()
+    near = [[0.0, 0.0, 0.0], [2.0, 2.0, 2.0]]
+    far = [[0.0, 0.0, 0.0], [4.0, 4.0, 4.0]]
+    for pts, want in ((near, 38), (far, 0), ([], 0)):
+        forms = [pts, np.array(pts, np.float32).reshape(-1, 3), torch.tensor(pts).reshape(-1, 3),
+                 torch.tensor(pts, dtype=torch.bfloat16).reshape(-1, 3), torch.tensor(pts, dtype=torch.float64).reshape(-1, 3),
+                 torch.tensor(pts).reshape(-1, 3).requires_grad_(True)]
+        for src in forms:
+            assert P.source_schedule(src, grid) == want
+            assert P.source_schedule(src, None) == 0

@@ -32,6 +32,10 @@ from ._native import BatchConfig, BatchScene, LyemError, check, lib
 
 C0 = 299792458.0
 
+# Part of the key of a tuned choice: raised with each change of the batched kernel after which the fastest configuration
+# may be another.
+KERNEL_REVISION = 2
+
 # (frequencies per thread, sources per visibility item, blocks per SM).  Blocks per
 # SM 3, 4, 6 or 8 select kernel variants whose registers are capped for that
 # occupancy; 0 runs the uncapped variant with as many blocks as fit.
@@ -292,10 +296,12 @@ class BatchedScattering:
 
     # ------------------------------------------------------------ autotuner
 
-    def signature(self, cell_scales=None):
+    def signature(self, cell_scales=None, candidates=None):
         sizes = [(d.src.shape[0], d.scat.shape[0], d.n_tris) for d in self.data]
         mode = list(cell_scales) if cell_scales else [round(c, 6) for c in self.grid_cells()]
-        h = hashlib.sha1(json.dumps([sizes, self.n_snk, self.n_freq, self.uniform, self.cull, mode]).encode())
+        cands = sorted({tuple(int(x) for x in c) for c in (candidates or CANDIDATES)})
+        h = hashlib.sha1(json.dumps([sizes, self.n_snk, self.n_freq, self.uniform, self.cull, mode, cands,
+                                     KERNEL_REVISION]).encode())
         return f"{torch.cuda.get_device_name(self.device)}|{h.hexdigest()}"
 
     def autotune(self, candidates=None, reps=1, use_cache=True, log=None, proxy=None, cell_scales=None):
@@ -304,7 +310,7 @@ class BatchedScattering:
         e.g. a cost-stratified subset of the scenes), keeps the fastest for this batch and
         returns {config: ms}.  With cell_scales, each scale of the density rule for the grid
         cells (set_cell_scale) is tried with every candidate, and the keys are config + (scale,)."""
-        key = self.signature(cell_scales)
+        key = self.signature(cell_scales, candidates)
         path = _cache_path()
         cache = {}
         if use_cache and os.path.exists(path):

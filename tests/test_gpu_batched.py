@@ -184,6 +184,22 @@ def test_autotune_picks_and_caches(small, tmp_path, monkeypatch):
     assert P.device_errors() == (0, 0)
 
 
+def test_autotune_cache_is_of_these_candidates_and_this_kernel(small, tmp_path, monkeypatch):
+    """A choice that was made among other candidates, or timed on another revision of the kernel, is not taken."""
+    B, P, _ = _mods()
+    scenes, snk, snk_n, freqs, ref, _ = small
+    monkeypatch.setenv("LYEM_TUNE_CACHE", str(tmp_path / "tune.json"))
+    bs = B.BatchedScattering(scenes, snk, snk_n, freqs)
+    assert set(bs.autotune(candidates=[(2, 64, 8)])) == {(2, 64, 8)}
+    assert set(bs.autotune(candidates=[(1, 32, 4), (4, 32, 4)])) == {(1, 32, 4), (4, 32, 4)}
+    assert bs.config in ((1, 32, 4), (4, 32, 4))
+    assert list(bs.autotune(candidates=[(4, 32, 4), (1, 32, 4)])) == [bs.config]  # the same ones: from the cache
+    monkeypatch.setattr(B, "KERNEL_REVISION", B.KERNEL_REVISION + 1)
+    assert len(bs.autotune(candidates=[(1, 32, 4), (4, 32, 4)])) == 2
+    assert _check(bs.run().cpu().numpy(), ref) < FIELD_TOL
+    assert P.device_errors() == (0, 0)
+
+
 def test_density_cells_same_field(small, tmp_path, monkeypatch):
     """Density-scaled grids (one scale for the batch, a cell per scene) change only the traversal
     work: the same visible paths and fields as the oracle; the autotuner picks a scale."""

@@ -796,33 +796,37 @@ __global__ void __launch_bounds__(kThreads, 16) grid_transposed_kernel(const Sta
     }
 }
 
-// Sums of the chunks' partial sums in FP64: a thread per element and eighth of the chunks, the eighths added in order.
-// One thread per element left the loads of its chunks one behind the other: 15,984 elements of 64 chunks 16.7 -> 8.3 us.
-constexpr int kReduceParts = 8;
+// Sums of the chunks' partial sums in FP64: PARTS threads per element, each a run of the chunks, the runs added in order.
+// One thread per element leaves the loads of its chunks one behind the other, eight per element leave most of a block
+// idle where there are few chunks.
+template <int PARTS>
 __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, long long n_chunks,
                                                              long long n_elem, float* __restrict__ out, int accumulate,
                                                              const int* __restrict__ choice, long long chosen_chunks) {
+    constexpr int kWidth = 256 / PARTS;
+    __shared__ double s_part[PARTS][kWidth];
     if (choice && *choice) n_chunks = chosen_chunks;
-    __shared__ double s_part[kReduceParts][32];
-    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
-    const long long per = (n_chunks + kReduceParts - 1) / kReduceParts;
+    const int slot = threadIdx.x % kWidth, part = threadIdx.x / kWidth;
+    const long long per = (n_chunks + PARTS - 1) / PARTS;
     const long long c0 = part * per, c1 = c0 + per < n_chunks ? c0 + per : n_chunks;
-    for (long long base = (long long)blockIdx.x * 32; base < n_elem; base += (long long)gridDim.x * 32) {
-        const long long i = base + lane;
-        double s = 0.0;
+    for (long long base = (long long)blockIdx.x * kWidth; base < n_elem; base += (long long)gridDim.x * kWidth) {
+        const long long i = base + slot;
+        double s = PARTS == 1 && accumulate && i < n_elem ? (double)out[i] : 0.0;
         if (i < n_elem) {
 #pragma unroll 8
             for (long long c = c0; c < c1; ++c) s += (double)partial[c * n_elem + i];
         }
-        s_part[part][lane] = s;
-        __syncthreads();
-        if (part == 0 && i < n_elem) {
-            s = accumulate ? (double)out[i] : 0.0;
+        if (PARTS > 1) {
+            s_part[part][slot] = s;
+            __syncthreads();
+            if (part == 0 && i < n_elem) {
+                s = accumulate ? (double)out[i] : 0.0;
 #pragma unroll
-            for (int k = 0; k < kReduceParts; ++k) s += s_part[k][lane];
-            out[i] = (float)s;
+                for (int k = 0; k < PARTS; ++k) s += s_part[k][slot];
+            }
         }
-        __syncthreads();
+        if (part == 0 && i < n_elem) out[i] = (float)s;
+        if (PARTS > 1) __syncthreads();
     }
 }
 
@@ -951,8 +955,17 @@ cudaError_t launch_reduce_partials(const float* partial, long long n_chunks, lon
                                    long long chosen_chunks) {
     const long long n_elem = 6 * n_snk;
     if (n_elem == 0) return cudaSuccess;
-    const unsigned blocks = capped_blocks(n_elem, 32, 64);
-    reduce_partials_kernel<<<blocks, 256, 0, stream>>>(partial, n_chunks, n_elem, out, accumulate, choice, chosen_chunks);
+    // Eight threads per element where one each are too few threads for the chunks' loads: at 1 / 8 / 64 / 512 chunks, us
+    // with one and with eight, 15,984 elements 5.7 / 6.4 / 20 / 121 and 5.6 / 5.8 / 10 / 45, 98,826 elements 5.6 / 8.5 /
+    // 34 / 230 and 9.8 / 12 / 31 / 198, 392,046 elements 7.7 / 18 / 107 / 813 and 22 / 30 / 105 / 745, 6,000,000 elements
+    // 40 / 194 / 1,431 and 217 / 356 / 1,525.
+    const long long chunks = n_chunks > chosen_chunks ? n_chunks : chosen_chunks;
+    if (n_elem <= 2048 * (chunks > 8 ? chunks : 8))
+        reduce_partials_kernel<8><<<capped_blocks(n_elem, 32, 64), 256, 0, stream>>>(partial, n_chunks, n_elem, out,
+                                                                                    accumulate, choice, chosen_chunks);
+    else
+        reduce_partials_kernel<1><<<capped_blocks(n_elem, 256, 16), 256, 0, stream>>>(partial, n_chunks, n_elem, out,
+                                                                                     accumulate, choice, chosen_chunks);
     note_launches(1);
     return cudaGetLastError();
 }

@@ -984,6 +984,26 @@ def test_device_arrays_enqueue_without_a_wait(n_src, n_snk):
     _no_device_errors()
 
 
+@pytest.mark.parametrize("n_src,n_snk", [(1, 1), (1, 2730), (1, 2731), (8, 2730), (9, 3072), (9, 3073), (70, 23893), (70, 23894),
+                                          (3, 200001)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_chunk_sums_both_reductions(n_src, n_snk, accumulate):
+    """The sum over source chunks at the edges of its rule (6 values a sink against 2,048 a chunk), one source a chunk: the
+    FP64 sum of the pairs, rounded once."""
+    P = _P()
+    src, snk, snk_n, v, f, E = random_scene(n_src, n_src=n_src, n_snk=n_snk, n_tris=3)
+    tris = P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f))
+    out = torch.full((n_snk, 3), 0.25 - 3j, dtype=torch.complex64, device="cuda") if accumulate else None
+    r = P.pair_stage(src, E, snk, snk_n, beta=30.0, tris=tris, self_to_self=True, want_pairs=True, src_chunk=1,
+                     sink_out=out, accumulate=accumulate)
+    pairs = torch.view_as_real(r.pairs).double()
+    want = pairs.sum(0) + (torch.tensor([0.25, -3.0], device="cuda") if accumulate else 0.0)
+    got = torch.view_as_real(r.sink).double()
+    # half an ulp, and the order of the FP64 sums
+    assert ((got - want).abs() <= 2.0 ** -24 * want.abs() + 1e-13 * (pairs.abs().sum(0) + 3)).all()
+    _no_device_errors()
+
+
 def test_scene_cache_reuses_device_grid():
     """Repeated model calls on the same solid reuse its device triangles and grid; the results are
     identical and a different solid builds a new scene."""

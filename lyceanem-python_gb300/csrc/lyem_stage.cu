@@ -9,7 +9,7 @@
 // network (the reference's output layout) and a visibility bit mask.
 //
 // Brute force (replaces raycast_brute_force, lyceanem/src/raycasting_brute_force.cuh:68-88):
-// triangle tiles of 128 are staged in shared memory by TMA bulk copies
+// triangle tiles of 128 (of 32 in the variant for few triangles) are staged in shared memory by TMA bulk copies
 // (double-buffered, mbarrier-completed, bounded waits).  For each source of the chunk a warp takes 32
 // triangles at a time, a lane each: it derives the ray-independent part of the test (tvec, qvec, e2.qvec) and drops
 // the triangles that face away from the source or that the beam of the warp's 32 rays cannot meet; its rays then test
@@ -121,6 +121,12 @@ constexpr int kThreads = 128;
 // Brute-force triangle tile (a power of two; two block barriers a tile): 32 / 64 / 128 / 256 / 512 triangles measured
 // 0.270 / 0.256 / 0.240 / 0.275 / 0.327 ms on the 8 x 8-array direct scene.
 constexpr int kTile = 128;
+// Triangles from which on the variant with beams runs.  Below, a ray tests them all as they lie in shared memory: a beam
+// costs about as much as a dozen tests.  1,024 sources to 16,471 sinks without / with beams 0.455 / 0.523 ms at 2 triangles,
+// 0.747 / 0.774 at 8, 0.796 / 0.770 at 16; two-sided 0.774 / 0.811 at 8, 0.828 / 0.872 at 20, 0.909 / 0.876 at 24.  64 to
+// 1,000,000 at 2 triangles 1.47 / 1.83.
+constexpr int kBeamTris = 16, kBeamTrisTwoSided = 24;
+constexpr int kFewTile = 32;  // tile of the variant without beams: all of its triangles
 constexpr int kBruteMaxChunk = 32;  // one bit per source in a 32-bit mask
 constexpr int kGridMaxChunk = 64;   // one bit per source in a 64-bit mask
 
@@ -129,9 +135,11 @@ int brute_max_src_chunk() { return kBruteMaxChunk; }
 int grid_max_src_chunk() { return kGridMaxChunk; }
 int transposed_src_chunk() { return 32; }
 
+template <bool BEAMS>
 struct BruteSmem {
-    float4 raw[2][kTile * 3];
-    TriPre pre[kThreads / 32][32];  // a warp's candidates of the current 32 triangles
+    static constexpr int kTris = BEAMS ? kTile : kFewTile;
+    float4 raw[2][kTris * 3];
+    TriPre pre[BEAMS ? kThreads / 32 : 1][BEAMS ? 32 : 1];  // a warp's candidates of the current 32 triangles
     unsigned long long mbar[2];
 };
 
@@ -313,10 +321,11 @@ __device__ __forceinline__ bool beam_misses(const BruteBeam& B, const TriPre& p)
 // triangles).  Against tests of every triangle by every ray: 64 sources, 2,664 sinks, 1,024 triangles 0.279 -> 0.240 ms
 // with the sinks in their natural order, 0.161 in direction order (two-sided test 0.620 -> 0.447 / 0.277); 256 sources,
 // 16,380 sinks 3.89 -> 1.67 / 1.23.
-template <bool CULL, bool WEIGHTED, bool PAIR_OUT, bool MASK_OUT>
+template <bool CULL, bool WEIGHTED, bool PAIR_OUT, bool MASK_OUT, bool BEAMS>
 __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StageParams p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    BruteSmem& sm = *reinterpret_cast<BruteSmem*>(smem_raw);
+    constexpr int kTris = BruteSmem<BEAMS>::kTris;
+    BruteSmem<BEAMS>& sm = *reinterpret_cast<BruteSmem<BEAMS>*>(smem_raw);
 
     const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -339,7 +348,7 @@ __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StagePar
         if (m_ok && !(p.skip_diag && src_index(s) == m)) pending |= 1u << s;
 
     const long long T = p.n_tris;
-    const int ntiles = (int)((T + kTile - 1) / kTile);
+    const int ntiles = (int)((T + kTris - 1) / kTris);
     const uint32_t mb0 = smem_addr(&sm.mbar[0]), mb1 = smem_addr(&sm.mbar[1]);
     if (tid == 0) {
         mbar_init(mb0, 1);
@@ -348,8 +357,8 @@ __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StagePar
     }
     __syncthreads();
     auto issue = [&](int k) {
-        long long first = (long long)k * kTile;
-        long long cnt = T - first < kTile ? T - first : kTile;
+        long long first = (long long)k * kTris;
+        long long cnt = T - first < kTris ? T - first : kTris;
         tma_load_1d(smem_addr(&sm.raw[k & 1][0]), p.tris + 3 * first, (uint32_t)(cnt * 48), (k & 1) ? mb1 : mb0);
     };
     int issued = ntiles < 2 ? ntiles : 2;
@@ -366,9 +375,9 @@ __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StagePar
     if (nsrc == 1) {
         const float* so = p.src_pos + 3 * src_index(0);
         r1 = vis_ray<CULL>(so[0], so[1], so[2], ex, ey, ez);
-        b1 = brute_beam(r1, pending & 1u);
+        if (BEAMS) b1 = brute_beam(r1, pending & 1u);
     }
-    TriPre* pre = sm.pre[tid >> 5];
+    TriPre* pre = sm.pre[BEAMS ? tid >> 5 : 0];
     int k = 0;
     for (; k < ntiles; ++k) {
         if (!__syncthreads_or(pending != 0)) break;
@@ -382,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StagePar
         }
         bool ok = mbar_wait_bounded((k & 1) ? mb1 : mb0, (k >> 1) & 1, kWaitCycles);
         if (__syncthreads_or(!ok)) { timed_out = true; break; }
-        const int cnt = (int)(T - (long long)k * kTile < kTile ? T - (long long)k * kTile : kTile);
+        const int cnt = (int)(T - (long long)k * kTris < kTris ? T - (long long)k * kTris : kTris);
         const float4* rt = sm.raw[k & 1];
         for (int s = 0; s < nsrc; ++s) {
             bool open = (pending >> s) & 1u;
@@ -393,9 +402,15 @@ __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StagePar
             BruteBeam beam = b1;
             if (nsrc > 1) {
                 r = vis_ray<CULL>(ox, oy, oz, ex, ey, ez);
-                beam = brute_beam(r, open);
+                if (BEAMS) beam = brute_beam(r, open);
             }
-            for (int base = 0; base < cnt; base += 32) {
+            if (!BEAMS && open) {
+                int j = 0;
+                while (j < cnt && !hit_full<CULL>(r, ox, oy, oz, rt[3 * j], rt[3 * j + 1], rt[3 * j + 2], p.eps)) ++j;
+                open = j == cnt;
+                tests += open ? cnt : j + 1;
+            }
+            for (int base = 0; BEAMS && base < cnt; base += 32) {
                 const int j = base + lane;
                 bool keep = j < cnt;
                 if (keep) {
@@ -920,8 +935,10 @@ static cudaError_t launch_t(const StageParams& p0, cudaStream_t stream) {
                 grid_stage_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, kLockstep><<<grid, kThreads, 0, stream>>>(p);
             note_launches(1);
         } else {
-            const size_t smem = sizeof(BruteSmem);
-            auto kern = brute_stage_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT>;
+            const bool beams = p.n_tris >= (CULL ? kBeamTris : kBeamTrisTwoSided);
+            const size_t smem = beams ? sizeof(BruteSmem<true>) : sizeof(BruteSmem<false>);
+            auto kern = beams ? brute_stage_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, true>
+                              : brute_stage_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, false>;
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
             kern<<<grid, kThreads, smem, stream>>>(p); note_launches(1);

@@ -148,6 +148,16 @@ def _check_buffer(name, t, dtype, n, exact):
         raise ValueError(f"{name} has {t.numel()} entries, {'' if exact else 'at least '}{n} needed")
 
 
+def _brute_order_pays(n_src, n_snk, n_tris, cull=True):
+    """Whether brute force without a given sink order should put the sinks in direction order from the first source.  A
+    warp then drops more triangles for its rays, which saves 0.2 to 0.4 us per million source-sink-triangle triples (twice
+    that in the two-sided test), but only where there are triangles to drop: from 24 on.  The order costs 0.02 ms up to
+    16,384 sinks (sorted in one block) and 0.1 ms and more above.  Unordered / ordered in ms: 1,024 sources to 2,664 sinks, 32
+    triangles 0.232 / 0.231, 48 0.255 / 0.243; 64 to 65,341, 48 0.315 / 0.364 (two-sided 0.478 / 0.382), 64 0.373 / 0.361, 96
+    0.447 / 0.371; 256 to 100,000, 2 0.72 / 0.85, 24 1.22 / 1.19, 48 1.37 / 1.21."""
+    return n_tris >= 24 and n_src * n_snk * n_tris * (1 if cull else 2) >= (130e6 if n_snk <= 16384 else 250e6)
+
+
 def pair_stage(src_pos, src_E, snk_pos, snk_nrm, *, beta, alpha=0.0, tris=None, grid=None, src_W=None,
                self_to_self=False, cull=True, eps=EPSILON, sink_out=None, accumulate=False, want_pairs=False,
                want_mask=False, counters=None, src_visible=None, snk_visible=None, src_order=None, snk_order=None,
@@ -199,10 +209,8 @@ def pair_stage(src_pos, src_E, snk_pos, snk_nrm, *, beta, alpha=0.0, tris=None, 
         T = tri_t.shape[0]
         cs = ct = cb = None
         org, cell, dims = f32arr([0, 0, 0]), 1.0, i32arr([1, 1, 1])
-        # a warp drops the triangles outside its rays' beam: from about 1.3e8 pairs x triangles on, sinks in direction
-        # order from the first source gain more than the order costs (64 sources, 2,664 sinks, 1,024 triangles: 0.24
-        # against 0.16 + 0.03 ms).  Results do not depend on the order.
-        if snk_order is None and N * M * T >= 1 << 27:
+        # results do not depend on the order
+        if snk_order is None and _brute_order_pays(N, M, T, cull):
             snk_order = torch.empty(M, dtype=torch.int32, device=dev)
             ws = _ws(lib.lyem_spatial_order_workspace(M), dev)
             check(lib.lyem_direction_order_from(_p(tp), M, _p(sp), _p(snk_order), _p(ws), ws.numel(), _stream()),

@@ -541,6 +541,82 @@ def test_brute_force_beam_culling(n_src, n_snk, n_tris, cull, spread):
     _no_device_errors()
 
 
+@pytest.mark.parametrize("n_src,n_snk", [(1, 33), (40, 97)])
+@pytest.mark.parametrize("n_tris", [1, 2, 15, 16, 17])
+@pytest.mark.parametrize("cull", [True, False])
+def test_brute_force_few_triangles(n_src, n_snk, n_tris, cull):
+    """Either side of the number of triangles from which on warps form beams, blocked and open rays, and coincident end
+    points: masks, counters and the field's visible sums equal to the oracle's."""
+    P = _P()
+    src, snk, snk_n, v, f, E = random_scene(n_src * 7 + n_tris, n_src=n_src, n_snk=n_snk, n_tris=n_tris)
+    v = (v * np.float32(3)).astype(np.float32)  # large triangles: some block
+    snk[n_snk // 2] = src[0]
+    tris = P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f))
+    kw = dict(self_to_self=True, cull=cull, eps=1e-6 if cull else 1e-7)
+    ot = O.pack_triangles(v, f)
+    om = O.mask_brute(src, snk, ot, **kw)
+    cnt = torch.zeros(2, dtype=torch.int64, device="cuda")
+    r = P.pair_stage(src, E, snk, snk_n, beta=30.0, tris=tris, want_mask=True, counters=cnt, **kw)
+    assert np.array_equal(r.mask().cpu().numpy(), om)
+    # a ray's tests: up to its first hit in triangle order, all where it is open
+    first = np.full((n_src, n_snk), n_tris)
+    for k in range(n_tris - 1, -1, -1):
+        first[~O.mask_brute(src, snk, ot[k:k + 1], **kw)] = k + 1
+    assert cnt.tolist() == [int(om.sum()), int(first.sum())]
+    _no_device_errors()
+
+
+def test_brute_force_order_only_where_it_pays():
+    """No order is made for a few triangles, however many pairs there are (it cannot drop what is not there), nor for a
+    small stage; results are those of the natural order."""
+    P = _P()
+    n_src, n_snk = 300, 50000
+    src, snk, snk_n, v, f, E = random_scene(11, n_src=n_src, n_snk=n_snk, n_tris=64)
+    src, snk, snk_n, E = (torch.from_numpy(x).cuda() for x in (src, snk, snk_n, E))
+    natural = torch.arange(n_snk, dtype=torch.int32, device="cuda")
+    for n_tris, launches in ((2, 2), (23, 2), (64, None)):
+        tris = P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f[:n_tris]))
+        before = P.kernel_launches()
+        r = P.pair_stage(src, E, snk, snk_n, beta=30.0, tris=tris, want_mask=True)
+        made = P.kernel_launches() - before
+        assert made == launches if launches else made > 2  # the stage and its sum; the order's sort besides
+        o = P.pair_stage(src, E, snk, snk_n, beta=30.0, tris=tris, want_mask=True, snk_order=natural)
+        assert torch.equal(o.mask_bits, r.mask_bits) and torch.equal(torch.view_as_real(o.sink), torch.view_as_real(r.sink))
+    few = P.pair_stage(src[:3], E[:3], snk[:100], snk_n[:100], beta=30.0, tris=tris)
+    before = P.kernel_launches()
+    again = P.pair_stage(src[:3], E[:3], snk[:100], snk_n[:100], beta=30.0, tris=tris)
+    assert P.kernel_launches() - before == 2 and torch.equal(torch.view_as_real(few.sink), torch.view_as_real(again.sink))
+    _no_device_errors()
+
+
+@pytest.mark.parametrize("n", [1, 33, 5000, 16385])
+def test_direction_order_from_a_device_point(n):
+    """The order seen from a point in device memory is that of the same point on the host, a non-finite point's one of the
+    indices all the same."""
+    import ctypes
+
+    from lyceanem_gb300 import _native
+    P = _P()
+    rng = np.random.default_rng(n)
+    pts = torch.from_numpy(rng.normal(size=(n, 3)).astype(np.float32)).cuda()
+    c = np.array([0.3, -0.2, 0.7], np.float32)
+    want = P.direction_order(pts, c)
+
+    def order(centre):
+        d = torch.from_numpy(centre).cuda()
+        out = torch.empty(n, dtype=torch.int32, device="cuda")
+        ws = torch.empty(_native.lib.lyem_spatial_order_workspace(n), dtype=torch.uint8, device="cuda")
+        _native.check(_native.lib.lyem_direction_order_from(
+            ctypes.c_void_p(pts.data_ptr()), n, ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(out.data_ptr()),
+            ctypes.c_void_p(ws.data_ptr()), ws.numel(), P._stream()), "direction_order_from")
+        return out
+    assert torch.equal(order(c), want)
+    for bad in (np.nan, np.inf):
+        got = order(np.array([bad, 0, 0], np.float32))
+        assert torch.equal(torch.sort(got.long()).values, torch.arange(n, device="cuda"))
+    _no_device_errors()
+
+
 def test_stage_buffer_checks():
     """Caller buffers of the wrong type or length are refused before any launch (the kernels index them
     without bounds checks)."""

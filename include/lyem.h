@@ -174,8 +174,9 @@ LYEM_API int lyem_spatial_order(const float *d_points, int64_t n_points, int32_t
  * the source arrays, and the rows left out are not written.  A source keeps
  * its row index, so self_to_self = 0 still skips the pair of equal row and
  * sink index.  Nothing checks the indices: each must be below the row count.
- * src_chunk: sources per thread block (0 = automatic; at most 32 for brute
- * force, 64 for the grid).  traversal (grid only): 1 = all lanes of a warp
+ * src_chunk: sources per thread block (at most 32 for brute force, 64 for the
+ * grid; 0 = automatic; grid: -1 / -2 = automatic for rays with short / long walks,
+ * a word that 0 finds from the grid's dimensions).  traversal (grid only): 1 = all lanes of a warp
  * trace the same source in lockstep; k in 2..33 = each lane moves on to its
  * next source when its ray ends, new rays being started in batches once k-1
  * lanes of the warp are idle; 34, 35, 36 = lockstep with the registers capped

@@ -121,21 +121,24 @@ struct DevBuf {
 
 void lyem::record_cuda_error(cudaError_t e) { g_last_cuda_error = (int)e; }
 
-// Sources per thread block when the caller passes 0.  Brute force: as many
-// as keep about four waves of blocks in flight (the triangle tiles are
+// Sources per thread block when the caller passes 0 or less.  Brute force: as
+// many as keep about four waves of blocks in flight (the triangle tiles are
 // re-staged per block).  Grid: 16, or 64 for 16,384 sources and more, fewer
-// when that would leave under eight waves of sixteen blocks an SM: the blocks
-// of a stage end at very different times (sinks over open ground, sinks behind
-// the clutter), and with one or two waves its last blocks run alone.  Lockstep,
-// with two waves -> with eight: 500 sources to 4,186 sinks 0.345 -> 0.326 ms,
-// 2,000 to 2,701 2.01 -> 1.51 (40,000 triangles), 2,000 to 4,186 1.13 -> 1.02,
-// 1,000 to 7,381 1.28 -> 1.05, 5,000 to 7,381 7.6 -> 7.2; 16 waves gain no more.
-// On the 28 GHz one-bounce scene the scatter->sink stage (50,000 sources)
-// measured 539.7 / 536.8 / 537.7 ms at 16 / 32 / 64, and 64 writes a quarter of
-// the per-chunk partial sums of 16; the 1,024-source stages were faster at 16.
-int lyem::auto_src_chunk(long long n_src, long long n_snk, bool grid) {
+// when that would leave too few blocks: the blocks of a stage end at very
+// different times (sinks over open ground, sinks behind the clutter), and with
+// one or two waves its last blocks run alone.  Where walks are long that wants
+// eight waves of sixteen blocks an SM, three where they are short and a block's
+// own work (its launch, its partial sums, 24 bytes a sink) counts.  Lockstep,
+// with two / three / eight waves: 1,000 sources to 7,381 sinks through 41 x 42 x 12
+// cells with 3.3 triangles each 2.23 / 1.90 / 1.81 ms, through 11 x 11 x 3 with 77
+// 6.63 / 5.58 / 5.03, through 4 x 4 x 1 with one 0.37 / 0.39 / 0.45; 64 to 65,341
+// through 11 x 10 x 3 with one 0.26 / 0.26 / 0.38; 2,000 to 2,701 through 15 x 14 x 4 with
+// one 0.51 / 0.47 / 0.50.  On the 28 GHz one-bounce scene the scatter->sink stage
+// (50,000 sources) measured 539.7 / 536.8 / 537.7 ms at 16 / 32 / 64, and 64 writes a
+// quarter of the per-chunk partial sums of 16; the 1,024-source stages were faster at 16.
+int lyem::auto_src_chunk(long long n_src, long long n_snk, bool grid, int walks) {
     const long long tiles = (n_snk + stage_block_threads() - 1) / stage_block_threads();
-    const long long waves = (long long)device_sm_count() * (grid ? 16 * 8 : 8 * 4);
+    const long long waves = (long long)device_sm_count() * (!grid ? 8 * 4 : walks == kShortWalks ? 16 * 3 : 16 * 8);
     long long c;
     if (grid) {
         c = n_src >= 16384 ? 64 : 16;
@@ -147,6 +150,15 @@ int lyem::auto_src_chunk(long long n_src, long long n_snk, bool grid) {
     return (int)std::max(1LL, std::min(c, cap));
 }
 
+namespace {
+// The caller's word (-1 short, -2 long), else by the grid's size, of which a walk crosses a part: grids with one cell per
+// triangle have walks that pay for more blocks from about 80 cells on all edges together.
+int walks_of(int src_chunk, const int32_t* dims3) {
+    if (src_chunk < 0) return src_chunk == -1 ? kShortWalks : kLongWalks;
+    if (!dims3) return kLongWalks;  // (more blocks, the larger workspace)
+    return (long long)dims3[0] + dims3[1] + dims3[2] < 80 ? kShortWalks : kLongWalks;
+}
+}  // namespace
 
 extern "C" {
 
@@ -325,7 +337,7 @@ LYEM_API size_t lyem_pair_stage_workspace(int64_t n_src, int64_t n_snk, int64_t 
                                           int32_t src_chunk) {
     (void)n_tris;
     if (n_src <= 0 || n_snk <= 0) return 256;
-    int chunk = src_chunk > 0 ? src_chunk : auto_src_chunk(n_src, n_snk, use_grid != 0);
+    int chunk = src_chunk > 0 ? src_chunk : auto_src_chunk(n_src, n_snk, use_grid != 0, walks_of(src_chunk, nullptr));
     chunk = std::min(chunk, use_grid ? grid_max_src_chunk() : brute_max_src_chunk());
     return stage_ws_bytes(n_src, n_snk, chunk);
 }
@@ -361,7 +373,8 @@ LYEM_API int lyem_pair_stage(const float* d_src_pos, const float* d_src_E, const
     if (((uintptr_t)d_src_E & 7u) || ((uintptr_t)d_src_W & 7u) || ((uintptr_t)d_pair_out & 7u) ||
         ((uintptr_t)d_sink_out & 7u))
         return LYEM_ERR_INVALID;
-    int chunk = src_chunk > 0 ? src_chunk : auto_src_chunk(n_src, n_snk, use_grid);
+    int chunk = src_chunk > 0 ? src_chunk
+                              : auto_src_chunk(n_src, n_snk, use_grid, walks_of(src_chunk, use_grid ? grid_dims3 : nullptr));
     chunk = std::min(chunk, use_grid ? grid_max_src_chunk() : brute_max_src_chunk());
     if (use_grid && traversal == 38) chunk = transposed_src_chunk();  // one lane per source of a chunk
     // 39: the lockstep and the transposed schedule are both launched, and the one that the sources' extent, found on the

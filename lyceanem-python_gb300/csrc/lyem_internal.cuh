@@ -98,8 +98,10 @@ cudaError_t launch_source_choice(const float* src_pos, const int* src_order, lon
                                  cudaStream_t stream);
 constexpr double kCompactCells = 4.0;  // (propagation.source_schedule: host arrays)
 int stage_block_threads();
-// Sources per thread block of a pair stage when the caller passes 0 (lyem_capi.cu).
-int auto_src_chunk(long long n_src, long long n_snk, bool grid);
+// Sources per thread block of a pair stage when the caller leaves them to the library (lyem_capi.cu); walks: what the
+// rays' walks take (grid only).
+constexpr int kShortWalks = 1, kLongWalks = 2;
+int auto_src_chunk(long long n_src, long long n_snk, bool grid, int walks = kLongWalks);
 int brute_max_src_chunk();
 int grid_max_src_chunk();
 int transposed_src_chunk();  // sources per block of the transposed grid schedule (traversal 38)

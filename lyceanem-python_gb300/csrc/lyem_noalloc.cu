@@ -39,19 +39,21 @@ int scratch_address(void** out) {
     return LYEM_OK;
 }
 
-// Source chunk for the fixed scratch: the caller's chunk, else the automatic
-// one when its partial sums fit, else the smallest larger chunk whose partial
-// sums fit; 0 when even the largest chunk's do not.
+// Source chunk for the fixed scratch: the caller's, which may be an automatic
+// one (0 or less) when its partial sums fit, else the smallest larger chunk whose
+// partial sums fit; kNoChunk when even the largest chunk's do not.
+constexpr int32_t kNoChunk = INT32_MIN;
 int32_t noalloc_chunk(int64_t n_src, int64_t n_snk, bool use_grid, int32_t src_chunk) {
     const int32_t cap = use_grid ? lyem::grid_max_src_chunk() : lyem::brute_max_src_chunk();
     if (src_chunk > 0) return src_chunk < cap ? src_chunk : cap;
-    const int32_t automatic = lyem::auto_src_chunk(n_src, n_snk, use_grid);
+    const int32_t automatic = lyem::auto_src_chunk(n_src, n_snk, use_grid, src_chunk == -1 ? lyem::kShortWalks : lyem::kLongWalks);
     // lyem_pair_stage's workspace: ceil(n_src / chunk) * n_snk * 24 bytes + 256
     const long long max_chunks = (long long)((kNoallocScratchBytes - 256) / (24ull * (unsigned long long)n_snk));
-    if (max_chunks < 1) return 0;
+    if (max_chunks < 1) return kNoChunk;
     const long long need = (n_src + max_chunks - 1) / max_chunks;
     const long long chunk = need > automatic ? need : automatic;
-    return chunk <= cap ? (int32_t)chunk : 0;
+    if (need <= automatic) return src_chunk;  // whatever lyem_pair_stage takes
+    return chunk <= cap ? (int32_t)chunk : kNoChunk;
 }
 
 }  // namespace
@@ -76,7 +78,7 @@ LYEM_API int lyem_pair_stage_noalloc(const float* d_src_pos, const float* d_src_
     int32_t chunk = src_chunk;
     if (n_src > 0 && n_snk > 0) {
         chunk = noalloc_chunk(n_src, n_snk, use_grid, src_chunk);
-        if (chunk <= 0 || lyem_pair_stage_workspace(n_src, n_snk, n_tris, use_grid, chunk) > kNoallocScratchBytes)
+        if (chunk == kNoChunk || lyem_pair_stage_workspace(n_src, n_snk, n_tris, use_grid, chunk) > kNoallocScratchBytes)
             return LYEM_ERR_WORKSPACE;
     }
     void* scratch = nullptr;

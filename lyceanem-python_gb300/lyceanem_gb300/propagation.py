@@ -110,6 +110,10 @@ class UniformGrid:
         check(lib.lyem_grid_fill(_p(tris), T, f32arr(self.origin), self.cell, i32arr(self.dims), _p(offsets),
                                  self.n_refs, _p(self.cell_start), _p(self.cell_tris), _p(self.cell_box), _p(ws2),
                                  ws2.numel(), _stream()), "grid_fill")
+        # Whether rays' walks are long or short, for the automatic source chunk: (cells on the edges)^2 x triangles a cell.
+        # Of 21 grids of 12 to 20,000 triangles and 0.25 to 5 m cells, those up to 8,400 were up to 45 % faster with the
+        # fewer blocks of short walks (at most 4 % slower), those from 17,000 on up to 13 % faster with those of long ones.
+        self.auto_chunk = -2 if sum(self.dims) ** 2 * self.n_refs >= 12000 * ncells else -1
         self._org_c = f32arr(self.origin)
         self._dims_c = i32arr(self.dims)
 
@@ -202,6 +206,7 @@ def pair_stage(src_pos, src_E, snk_pos, snk_nrm, *, beta, alpha=0.0, tris=None, 
     if grid is not None:
         tri_t, T = None, 0
         cs, ct, cb = grid.cell_start, grid.cell_tris, grid.cell_box
+        src_chunk = src_chunk or getattr(grid, "auto_chunk", 0)
         org, cell, dims = grid._org_c, grid.cell, grid._dims_c
     else:
         tri_t = _dev(tris, torch.float32).reshape(-1, 12).contiguous() if tris is not None else \

@@ -1080,6 +1080,33 @@ def test_chunk_sums_both_reductions(n_src, n_snk, accumulate):
     _no_device_errors()
 
 
+@pytest.mark.parametrize("n_src,n_snk", [(1, 1), (33, 500), (1000, 7381), (64, 20011)])
+@pytest.mark.parametrize("cell", [None, 0.05])
+def test_automatic_chunk_by_length_of_walks(n_src, n_snk, cell):
+    """The automatic source chunk for short and for long walks, asked for and found from the grid: same masks and counts,
+    the field to rounding; short walks take no more blocks than long ones, far fewer where the stage is large enough."""
+    from lyceanem_gb300 import _native
+    P = _P()
+    src, snk, snk_n, v, f, E = random_scene(n_src, n_src=n_src, n_snk=n_snk, n_tris=150)
+    g = P.UniformGrid(P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f)), cell=cell)
+    if cell is None:
+        assert g.auto_chunk == -1
+    ws = [_native.lib.lyem_pair_stage_workspace(n_src, n_snk, 0, 1, c) for c in (-1, -2, 0)]
+    assert ws[0] <= ws[1] == ws[2]
+    if (n_src, n_snk) == (1000, 7381):
+        assert 2 * ws[0] <= ws[1] + 256
+    i32 = dict(dtype=torch.int32, device="cuda")
+    res = []
+    for c in (16, 0, -1, -2, -7):
+        sv, cnt = torch.zeros(n_src, **i32), torch.zeros(2, dtype=torch.int64, device="cuda")
+        r = P.pair_stage(src, E, snk, snk_n, beta=30.0, grid=g, want_mask=True, src_chunk=c, src_visible=sv, counters=cnt)
+        res.append((r.mask_bits, sv, cnt[:1], r.sink))
+    for m, sv, cnt, sink in res[1:]:
+        assert torch.equal(m, res[0][0]) and torch.equal(sv, res[0][1]) and torch.equal(cnt, res[0][2])
+        assert rel_err(sink.cpu().numpy(), res[0][3].cpu().numpy()) < 2e-6  # FP32 sums of up to 16 terms, then FP64
+    _no_device_errors()
+
+
 def test_scene_cache_reuses_device_grid():
     """Repeated model calls on the same solid reuse its device triangles and grid; the results are
     identical and a different solid builds a new scene."""

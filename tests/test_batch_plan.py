@@ -64,6 +64,22 @@ def test_item_counts(fg, chunk):
     assert ws >= bits + sum(Pn * F * 24 for _, Pn in sizes)
 
 
+def test_queries_do_not_make_the_list():
+    """Workspace and item queries (and the launch, which plans in the same way) only count: a batch of 6.7e7 visibility
+    items, whose list would take 1.1 GB, is answered at once, and one beyond 2^31 items is refused."""
+    import time
+    cfg = _cfg(fg=4, chunk=32)
+    scenes = (BatchScene * 1)(_scene(64, 1 << 20))
+    t = time.perf_counter()
+    ws = lib.lyem_batch_workspace(scenes, 1, 1 << 16, 4, ctypes.byref(cfg))
+    n = lib.lyem_batch_items(scenes, 1, 1 << 16, 4, ctypes.byref(cfg), None)
+    assert time.perf_counter() - t < 0.1
+    vis = 2 * _ceil(1 << 20, 32) + 2 * _ceil(1 << 16, 32) + _ceil(1 << 20, 32) * _ceil(1 << 16, 32)
+    assert n > vis and ws > 16 * vis
+    big = (BatchScene * 1)(_scene(64, 1 << 21))
+    assert lib.lyem_batch_workspace(big, 1, 1 << 22, 4, ctypes.byref(cfg)) == 0
+
+
 def test_rejects_bad_arguments():
     scenes = (BatchScene * 1)(_scene(64, 10))
     for cfg in (_cfg(fg=3), _cfg(chunk=48), _cfg(bps=9)):

@@ -167,6 +167,17 @@ def test_batched_vs_pair_stages():
     assert P.device_errors() == (0, 0)
 
 
+@pytest.mark.parametrize("config", [(4, 64, 8), (4, 32, 8), (4, 32, 3), (2, 32, 6), (1, 64, 8), (8, 64, 3)])
+def test_register_capped_variants_vs_oracle(small, config):
+    """The variants of the kernel that are capped for an occupancy give the oracle's field and visible pairs."""
+    B, P, _ = _mods()
+    scenes, snk, snk_n, freqs, ref, counts = small
+    bs = B.BatchedScattering(scenes, snk, snk_n, freqs, config=config)
+    assert _check(bs.run().cpu().numpy(), ref) < FIELD_TOL
+    assert np.array_equal(bs.counters.cpu().numpy()[:, :3], counts)
+    assert P.device_errors() == (0, 0)
+
+
 def test_autotune_picks_and_caches(small, tmp_path, monkeypatch):
     B, P, _ = _mods()
     scenes, snk, snk_n, freqs, ref, _ = small

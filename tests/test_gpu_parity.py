@@ -1034,6 +1034,7 @@ def test_schedule_chosen_on_the_device(n_src, n_snk, spread):
     _no_device_errors()
 
 
+@pytest.mark.filterwarnings("ignore:Synchronization debug mode")
 @pytest.mark.parametrize("n_src,n_snk", [(1024, 2000), (300, 4000), (20, 300)])
 def test_device_arrays_enqueue_without_a_wait(n_src, n_snk):
     """With device arrays, the network and the numba fields only enqueue work: no copy back, no synchronisation."""

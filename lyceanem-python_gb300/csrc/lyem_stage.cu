@@ -502,14 +502,16 @@ constexpr int kLockstep16 = 4;
 // longest ray of each source.
 constexpr int kTwoPhase16 = 5;
 constexpr int kTwoPhase12 = 6;
+// kLockstep16 for a launch that p.choice may turn off (a variant of its own: the test costs the walk a register).
+constexpr int kChosen16 = 7;
 
 // COUNT = false (only with the default schedule, when the caller asks for no
 // counters) leaves the per-test counting out of the walk: one instruction and
 // one register less in the innermost loop (scatter->sink stage of the 28 GHz
 // scene 448 -> 440 ms).
 template <bool CULL, bool WEIGHTED, bool PAIR_OUT, bool MASK_OUT, int MODE, bool COUNT = true>
-__global__ void __launch_bounds__(kThreads, MODE == kLockstep10 ? 10 : (MODE == kLockstep12 || MODE == kTwoPhase12) ? 12 : (MODE == kLockstep16 || MODE == kTwoPhase16) ? 16 : 1) grid_stage_kernel(const StageParams p) {
-    if (p.choice && *p.choice != p.choice_is) return;
+__global__ void __launch_bounds__(kThreads, MODE == kLockstep10 ? 10 : (MODE == kLockstep12 || MODE == kTwoPhase12) ? 12 : (MODE == kLockstep16 || MODE == kChosen16 || MODE == kTwoPhase16) ? 16 : 1) grid_stage_kernel(const StageParams p) {
+    if (MODE == kChosen16 && *p.choice != p.choice_is) return;
     // 32-bit indices (fewer live registers in the walk): the entry point keeps
     // n_src and n_snk below 2^31 - 256
     const int tid = threadIdx.x;
@@ -918,6 +920,12 @@ static cudaError_t launch_t(const StageParams& p0, cudaStream_t stream) {
                     grid_transposed_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, true><<<grid, kThreads, 0, stream>>>(p);
                 else
                     grid_transposed_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, false><<<grid, kThreads, 0, stream>>>(p);
+            } else if (p.refill_lanes == -16 && p.choice) {
+                if (p.counters)
+                    grid_stage_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, kChosen16><<<grid, kThreads, 0, stream>>>(p);
+                else
+                    grid_stage_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, kChosen16, false>
+                        <<<grid, kThreads, 0, stream>>>(p);
             } else if (p.refill_lanes == -16) {
                 if (p.counters)
                     grid_stage_kernel<CULL, WEIGHTED, PAIR_OUT, MASK_OUT, kLockstep16><<<grid, kThreads, 0, stream>>>(p);

@@ -110,10 +110,13 @@ class UniformGrid:
         check(lib.lyem_grid_fill(_p(tris), T, f32arr(self.origin), self.cell, i32arr(self.dims), _p(offsets),
                                  self.n_refs, _p(self.cell_start), _p(self.cell_tris), _p(self.cell_box), _p(ws2),
                                  ws2.numel(), _stream()), "grid_fill")
-        # Whether rays' walks are long or short, for the automatic source chunk: (cells on the edges)^2 x triangles a cell.
-        # Of 21 grids of 12 to 20,000 triangles and 0.25 to 5 m cells, those up to 8,400 were up to 45 % faster with the
-        # fewer blocks of short walks (at most 4 % slower), those from 17,000 on up to 13 % faster with those of long ones.
-        self.auto_chunk = -2 if sum(self.dims) ** 2 * self.n_refs >= 12000 * ncells else -1
+        # Whether rays' walks are long or short, for the automatic source chunk: by the cells they cross and by the triangles
+        # in these.  Of 21 grids of 12 to 20,000 triangles and 0.25 to 5 m cells, those of less than 80 cells on the edges
+        # and up to 8,400 in the product below were up to 45 % faster with the fewer blocks of short walks (at most 4 %
+        # slower); those of more cells were up to 13 % faster with the blocks of long ones, if mostly empty as well, and so
+        # were those from 17,000 on.
+        d = sum(self.dims)
+        self.auto_chunk = -2 if d >= 80 or d * d * self.n_refs >= 12000 * ncells else -1
         self._org_c = f32arr(self.origin)
         self._dims_c = i32arr(self.dims)
 

@@ -61,8 +61,9 @@ LYEM_API uint64_t lyem_kernel_launches(void);
  * FMA lane-operations per second, the denominator of the visibility roofline. */
 LYEM_API int lyem_fp32_fma_probe(int64_t iterations, double *fma_per_second, void *stream);
 /* Synchronises `stream`, then reads and clears the library's device error word
- * (bit 0: a bounded wait expired; the other bits are reserved).  Returns
- * LYEM_ERR_TIMEOUT if bit 0 was set. */
+ * (bit 0: a bounded wait expired; bit 1: an index out of range was found, by
+ * lyem_pack_triangles or in a path list).  Returns LYEM_ERR_TIMEOUT if bit 0 was
+ * set. */
 LYEM_API int lyem_device_errors(void *stream, uint32_t *flags_out);
 
 /* ---------------------------------------------------------------- geometry */
@@ -356,9 +357,9 @@ typedef struct lyem_batch_config {
  *   E_f(m) = sum_n S0_f(n, m) + sum_p e_p(f) (.) S2_f(p, m; e_p(f)),
  *   e_p(f) = sum_n S1_f(n, p).
  * lyem_batch_workspace: bytes of the workspace (0: invalid arguments).
- * lyem_batch_items: work items of the launch (per kind: three visibility
- *   stages, scatter fields, sink fields; a launch may take an item in
- *   parts), or minus a status.
+ * lyem_batch_items: the batch's work in nominal items (per kind: three
+ *   visibility stages, scatter fields, sink fields in runs of some 16,384
+ *   pairs), or minus a status.  The launch takes the same work in smaller parts.
  * lyem_batch_prepare: writes the scene table, the work list and the
  *   frequency tables into the workspace (256-byte aligned); host -> device
  *   copies, synchronous with the stream.  Repeat after any change of scenes,

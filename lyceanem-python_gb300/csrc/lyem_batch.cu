@@ -60,7 +60,7 @@ namespace {
 
 constexpr int kBT = 256;  // threads per block (8 independent warps)
 constexpr int kWarpSinks = 32;               // sinks of a visibility item (one per lane)
-constexpr long long kItemPairs = 1LL << 14;  // candidate pairs a field item should cover at least
+constexpr long long kItemPairs = 1LL << 14;  // pairs of a nominal field item (lyem_batch_items; the queue holds parts)
 constexpr int kKinds = 5;
 enum Kind { kVisScat = 0, kVisDirect = 1, kVisBounce = 2, kFieldW = 3, kFieldE = 4 };
 
@@ -758,9 +758,9 @@ int make_plan(const lyem_batch_scene* sc, int n_scenes, long long n_snk, int n_f
         add_vis(s, kVisDirect, N, n_snk);
         add_vis(s, kVisBounce, P, n_snk);
     }
-    // A field item is a run of 32-slot chunks (slot = point * groups + group),
-    // long enough for about kItemPairs candidate (pair, group) evaluations.
-    // The list holds its parts: a chunk each (more where a point has fewer
+    // The nominal field items, which lyem_batch_items reports, are runs of 32-slot
+    // chunks (slot = point * groups + group) of about kItemPairs candidate (pair,
+    // group) evaluations.  The list holds parts: a chunk each (more where a point has fewer
     // than 64 sources), or a point each (more where it has fewer than 512),
     // since a warp adds their pairs one behind the other whatever the number
     // of groups, and long runs left most warps without work.  8 scenes of up to 178 elements, 1,649 sinks, 8 / 64 frequencies:

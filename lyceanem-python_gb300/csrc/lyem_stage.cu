@@ -480,7 +480,8 @@ __global__ void __launch_bounds__(kThreads, 9) brute_stage_kernel(const StagePar
 //             warp are idle, or none is busy) so the set-up code is not
 //             serialised lane by lane.
 // Visibility of the chunk is kept as a 64-bit blocked mask; the field epilogue
-// then runs over the sources in lockstep.
+// then takes each lane from one of its own visible sources to the next, or, with
+// a per-pair output, all lanes through the sources in lockstep.
 constexpr int kLockstep = 0;
 constexpr int kRefill = 1;
 // Lockstep with the registers capped so that 10, 12 or 16 blocks of 128

@@ -237,8 +237,8 @@ class BatchedScattering:
         self.graph = None
 
     def items(self):
-        """Work items of the launch per kind: visibility (sources->scatter, sources->sinks,
-        scatter->sinks), scatter fields, sink fields."""
+        """The batch's work in nominal items per kind: visibility (sources->scatter, sources->sinks,
+        scatter->sinks), scatter fields, sink fields (the launch takes these in smaller parts)."""
         per = (ctypes.c_int64 * 5)()
         n = lib.lyem_batch_items(self._structs, self.n_scenes, self.n_snk, self.n_freq, ctypes.byref(self._cfg_c),
                                  per)

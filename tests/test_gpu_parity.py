@@ -1034,6 +1034,50 @@ def test_schedule_chosen_on_the_device(n_src, n_snk, spread):
     _no_device_errors()
 
 
+def test_schedule_chosen_for_each_replay():
+    """A captured network chooses its schedule when it is replayed: for the sources that are there then."""
+    from lyceanem_gb300 import beam_sweep as BS
+    P = _P()
+    src, snk, snk_n, v, f, E = random_scene(21, n_src=100, n_snk=3000, n_tris=100)
+    g = P.UniformGrid(P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f)))
+    near = torch.from_numpy((0.01 * src).astype(np.float32)).cuda()
+    far = torch.from_numpy((40 * src).astype(np.float32)).cuda()
+    snk, snk_n, E = (torch.from_numpy(x).cuda() for x in (snk, snk_n, E))
+    assert P.source_schedule(near.cpu(), g) == 38 and P.source_schedule(far.cpu(), g) == 0
+    want = [BS.form_network(s, E, snk, snk_n, beta=30.0, grid=g) for s in (near, far)]
+    held = near.clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = BS.form_network(held, E, snk, snk_n, beta=30.0, grid=g)
+    for k in (0, 1, 0):
+        held.copy_((near, far)[k])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(torch.view_as_real(out), torch.view_as_real(want[k]))
+    _no_device_errors()
+
+
+def test_network_into_a_given_tensor():
+    """pairs_out takes the network, with zeros in the rows that a subset leaves out; other forms are refused."""
+    P = _P()
+    src, snk, snk_n, v, f, E = random_scene(4, n_src=10, n_snk=70, n_tris=30)
+    g = P.UniformGrid(P.pack_triangles(torch.from_numpy(v), torch.from_numpy(f)))
+    kw = dict(beta=30.0, grid=g)
+    want = P.pair_stage(src, E, snk, snk_n, want_pairs=True, **kw).pairs
+    whole = torch.full((30, 70, 3), 9.0, dtype=torch.complex64, device="cuda")
+    r = P.pair_stage(src, E, snk, snk_n, pairs_out=whole[10:20], **kw)
+    assert r.pairs.data_ptr() == whole[10:20].data_ptr() and torch.equal(torch.view_as_real(whole[10:20]), torch.view_as_real(want))
+    assert bool((whole[:10] == 9).all()) and bool((whole[20:] == 9).all())
+    some = torch.tensor([7, 2], dtype=torch.int32, device="cuda")
+    P.pair_stage(src, E, snk, snk_n, pairs_out=whole[10:20], src_order=some, **kw)
+    assert torch.equal(torch.view_as_real(whole[12]), torch.view_as_real(want[2])) and not bool(whole[13].any())
+    for bad in (whole[:9], whole[:10].to(torch.complex128), whole[::3], whole[:10].cpu()):
+        with pytest.raises(ValueError):
+            P.pair_stage(src, E, snk, snk_n, pairs_out=bad, **kw)
+    _no_device_errors()
+
+
 @pytest.mark.filterwarnings("ignore:Synchronization debug mode")
 @pytest.mark.parametrize("n_src,n_snk", [(1024, 2000), (300, 4000), (20, 300)])
 def test_device_arrays_enqueue_without_a_wait(n_src, n_snk):
